@@ -20,6 +20,7 @@
 
 #include "../../include/mpm_b200.h"
 #include "mpm_kernels.cuh"
+#include "mpm_records.cuh"
 
 using namespace mpm;
 
@@ -77,6 +78,9 @@ struct SceneHost {
 
 }  // namespace
 
+constexpr int READBACK_FLAGS = 12;
+constexpr size_t P2G_RECORD_BYTES = 2 * sizeof(float4) + sizeof(float2) + sizeof(uint32_t);
+
 struct mpm_solver {
     int device = 0;
     cudaStream_t stream = nullptr;
@@ -105,7 +109,8 @@ struct mpm_solver {
     cudaEvent_t params_copied = nullptr;
     uint32_t *d_status = nullptr;    // scene 0's status words (in dyn)
     uint32_t *d_counters = nullptr;  // scene 0's counters (in dyn)
-    uint32_t *h_readback = nullptr;  // pinned: 2 counters + 8 status words (+ spare)
+    uint32_t *h_readback = nullptr;  // pinned: 2 counters + 8 status words; from READBACK_FLAGS on, flags
+                                     // that a kernel sets when it meets a record it cannot place
 
     ParticleBuffers buf[2]{};
     uint32_t *bonded = nullptr, *obj = nullptr;  // by original index
@@ -172,6 +177,14 @@ struct mpm_solver {
     std::map<std::tuple<int, int>, cudaGraphExec_t> graphs;
     // graphs of whole short batches: (substeps, start parity, guarded)
     std::map<std::tuple<uint32_t, int, int>, cudaGraphExec_t> batch_graphs;
+    // records between the host and the device: the device's pinned staging, and
+    // a slab of slab_records records with their object ids.  The P2G records,
+    // which every batch writes anew, share the slab's memory; tmp and keys serve
+    // as the slots of the original indices and the requested indices.
+    RecordStage *stage = nullptr;
+    unsigned char *slab = nullptr;
+    uint32_t slab_records = 0;
+
     // the last batch's graph copied the compact readback (counters and
     // status) to h_readback, and no call since could have changed them
     bool readback_ready = false;
@@ -717,104 +730,96 @@ uint32_t intern_material(std::vector<Material> &table, const float *w)
     return (uint32_t)(table.size() - 1);
 }
 
-// Uploads packed records in original order: slot i holds particle i.
-// Uploads `count` packed particles into slots slot_base.. of buffer `target`
-// as original indices orig_base..
-int unpack_and_upload(mpm_solver *s, const float *packed, uint32_t count, int target, uint32_t slot_base = 0,
-                      uint32_t orig_base = 0)
+// Ends the loan of a pinned chunk when its call returns.
+struct ReturnChunk {
+    mpm_solver *s;
+    bool lent;
+    ~ReturnChunk()
+    {
+        if (lent) s->stage->lend_end(s->stream);
+    }
+};
+
+// Checks `count` packed records in order and adds their materials to the
+// table in the order they first appear.
+int intern_materials(mpm_solver *s, const float *packed, uint32_t count)
 {
-    std::vector<float2> pos(count), vel(count);
-    std::vector<float4> C(count), F(count);
-    std::vector<float> pvol(count), damage(count), vol(count);
-    std::vector<uint32_t> mat(count), bonded(count), orig(count);
-    const size_t before = s->mats.size();
+    const float *last = nullptr;  // the last record looked up
     for (uint32_t i = 0; i < count; ++i) {
         const float *w = packed + (size_t)i * MPM_PARTICLE_WORDS;
-        const uint32_t model = f2u(w[13]);
+        const uint32_t model = f2u(w[13]), marker = f2u(w[19]);
         if (model > MODEL_FIXED_COROTATED)
             return set_error(MPM_ERR_INVALID_ARGUMENT, "particle %u has an unsupported MPM material model %u", i, model);
-        pos[i] = make_float2(w[0], w[1]);
-        vel[i] = make_float2(w[2], w[3]);
-        C[i] = make_float4(w[4], w[5], w[6], w[7]);
-        F[i] = make_float4(w[8], w[9], w[10], w[11]);
-        pvol[i] = w[12];
-        damage[i] = model == MODEL_NEO_HOOKEAN ? w[18] : 0.0f;
-        vol[i] = w[17];
-        mat[i] = intern_material(s->mats, w);
-        bonded[i] = f2u(w[19]);
-        orig[i] = orig_base + i;
-        if (bonded[i] > 3u) return set_error(MPM_ERR_INVALID_ARGUMENT, "particle %u has an invalid bonded triangle marker", i);
+        // words 13-16 and the parameter: the material of the record before it
+        if (!last || std::memcmp(last + 13, w + 13, 4 * sizeof(float)) != 0 || f2u(last[18]) != f2u(w[18])) {
+            intern_material(s->mats, w);
+            last = w;
+        }
+        if (marker > 3u) return set_error(MPM_ERR_INVALID_ARGUMENT, "particle %u has an invalid bonded triangle marker", i);
     }
     if (s->mats.size() > 65536) return set_error(MPM_ERR_INVALID_ARGUMENT, "more than 65536 distinct materials");
-    if (s->mats.size() != before || s->d_mats == nullptr) {
-        CUDA_TRY(cudaStreamSynchronize(s->stream));
-        if (s->d_mats) cudaFree(s->d_mats);
-        s->d_mats = nullptr;
-        CUDA_TRY(dalloc(&s->d_mats, s->mats.size()));
-        CUDA_TRY(cudaMemcpyAsync(s->d_mats, s->mats.data(), s->mats.size() * sizeof(Material), cudaMemcpyHostToDevice,
-                                 s->stream));
-        // captured graphs hold the old table pointer
-        drop_graphs(s);
-    }
-    ParticleBuffers &b = s->buf[target];
-    const size_t d = slot_base;
-    CUDA_TRY(cudaMemcpyAsync(b.pos + d, pos.data(), count * sizeof(float2), cudaMemcpyHostToDevice, s->stream));
-    CUDA_TRY(cudaMemcpyAsync(b.vel + d, vel.data(), count * sizeof(float2), cudaMemcpyHostToDevice, s->stream));
-    CUDA_TRY(cudaMemcpyAsync(b.C + d, C.data(), count * sizeof(float4), cudaMemcpyHostToDevice, s->stream));
-    CUDA_TRY(cudaMemcpyAsync(b.F + d, F.data(), count * sizeof(float4), cudaMemcpyHostToDevice, s->stream));
-    CUDA_TRY(cudaMemcpyAsync(b.pvol + d, pvol.data(), count * sizeof(float), cudaMemcpyHostToDevice, s->stream));
-    CUDA_TRY(cudaMemcpyAsync(b.damage + d, damage.data(), count * sizeof(float), cudaMemcpyHostToDevice, s->stream));
-    CUDA_TRY(cudaMemcpyAsync(b.vol + d, vol.data(), count * sizeof(float), cudaMemcpyHostToDevice, s->stream));
-    CUDA_TRY(cudaMemcpyAsync(b.mat + d, mat.data(), count * sizeof(uint32_t), cudaMemcpyHostToDevice, s->stream));
-    CUDA_TRY(cudaMemcpyAsync(b.orig + d, orig.data(), count * sizeof(uint32_t), cudaMemcpyHostToDevice, s->stream));
-    CUDA_TRY(cudaMemcpyAsync(s->bonded + orig_base, bonded.data(), count * sizeof(uint32_t), cudaMemcpyHostToDevice,
-                             s->stream));
-    if (s->slot_of[target]) {
-        // the uploaded slots are in original order
-        std::vector<uint32_t> slots(count);
-        for (uint32_t i = 0; i < count; ++i) slots[i] = slot_base + i;
-        CUDA_TRY(cudaMemcpyAsync(s->slot_of[target] + orig_base, slots.data(), count * sizeof(uint32_t),
-                                 cudaMemcpyHostToDevice, s->stream));
-        CUDA_TRY(cudaStreamSynchronize(s->stream));
-    }
-    // the copies above read pageable host vectors; wait before they go away
-    CUDA_TRY(cudaStreamSynchronize(s->stream));
     return MPM_OK;
 }
 
-// Copies the slot arrays of the current buffer to the host.
-struct HostState {
-    std::vector<float2> pos, vel;
-    std::vector<float4> C, F;
-    std::vector<float> pvol, damage, vol;
-    std::vector<uint32_t> mat, orig;
-};
-
-int download_state(mpm_solver *s, HostState &h)
+// Gives the device the material table after it grew (or at the start).
+int upload_materials(mpm_solver *s)
 {
-    const uint32_t n = s->n;
-    h.pos.resize(n);
-    h.vel.resize(n);
-    h.C.resize(n);
-    h.F.resize(n);
-    h.pvol.resize(n);
-    h.damage.resize(n);
-    h.vol.resize(n);
-    h.mat.resize(n);
-    h.orig.resize(n);
-    const ParticleBuffers &b = s->buf[s->cur];
-    if (n > 0) {
-        CUDA_TRY(cudaMemcpyAsync(h.pos.data(), b.pos, n * sizeof(float2), cudaMemcpyDeviceToHost, s->stream));
-        CUDA_TRY(cudaMemcpyAsync(h.vel.data(), b.vel, n * sizeof(float2), cudaMemcpyDeviceToHost, s->stream));
-        CUDA_TRY(cudaMemcpyAsync(h.C.data(), b.C, n * sizeof(float4), cudaMemcpyDeviceToHost, s->stream));
-        CUDA_TRY(cudaMemcpyAsync(h.F.data(), b.F, n * sizeof(float4), cudaMemcpyDeviceToHost, s->stream));
-        CUDA_TRY(cudaMemcpyAsync(h.pvol.data(), b.pvol, n * sizeof(float), cudaMemcpyDeviceToHost, s->stream));
-        CUDA_TRY(cudaMemcpyAsync(h.damage.data(), b.damage, n * sizeof(float), cudaMemcpyDeviceToHost, s->stream));
-        CUDA_TRY(cudaMemcpyAsync(h.vol.data(), b.vol, n * sizeof(float), cudaMemcpyDeviceToHost, s->stream));
-        CUDA_TRY(cudaMemcpyAsync(h.mat.data(), b.mat, n * sizeof(uint32_t), cudaMemcpyDeviceToHost, s->stream));
-        CUDA_TRY(cudaMemcpyAsync(h.orig.data(), b.orig, n * sizeof(uint32_t), cudaMemcpyDeviceToHost, s->stream));
-    }
     CUDA_TRY(cudaStreamSynchronize(s->stream));
+    if (s->d_mats) cudaFree(s->d_mats);
+    s->d_mats = nullptr;
+    CUDA_TRY(dalloc(&s->d_mats, s->mats.size()));
+    CUDA_TRY(cudaMemcpy(s->d_mats, s->mats.data(), s->mats.size() * sizeof(Material), cudaMemcpyHostToDevice));
+    // captured graphs hold the old table pointer
+    drop_graphs(s);
+    return MPM_OK;
+}
+
+// Uploads `count` packed particles into slots slot_base.. of buffer `target`
+// as original indices orig_base...  The records cross as they are and a kernel
+// unpacks them.  The host reads the records itself only when the table may
+// lack one of their materials: at the start, when k_check_records found one
+// that it does not hold (or an invalid one), or for uploads beyond one slab.
+int unpack_and_upload(mpm_solver *s, const float *packed, uint32_t count, int target, uint32_t slot_base = 0,
+                      uint32_t orig_base = 0)
+{
+    if (count == 0) return MPM_OK;
+    const size_t record = MPM_PARTICLE_WORDS * sizeof(float);
+    const bool one_slab = count <= s->slab_records;
+    // the kernels read what fits one chunk straight from pinned memory, the
+    // rest from the device slab
+    void *lent = s->stage->lend((size_t)count * record);
+    const ReturnChunk give_back{s, lent != nullptr};
+    float *const records = reinterpret_cast<float *>(lent ? lent : s->slab);
+    bool look = s->d_mats == nullptr || !one_slab;
+    if (lent)
+        std::memcpy(lent, packed, (size_t)count * record);
+    else if (one_slab)
+        CUDA_TRY(s->stage->copy_in(s->stream, records, packed, (size_t)count * record));
+    if (!look) {
+        volatile uint32_t *const flags = s->h_readback + READBACK_FLAGS;
+        flags[0] = 0u;
+        k_check_records<<<blocks_for(count, RECORD_THREADS), RECORD_THREADS, 0, s->stream>>>(
+            records, count, s->d_mats, (uint32_t)s->mats.size(), s->h_readback + READBACK_FLAGS);
+        CUDA_TRY(cudaGetLastError());
+        CUDA_TRY(cudaStreamSynchronize(s->stream));
+        look = flags[0] != 0u;
+    }
+    if (look) {
+        const size_t before = s->mats.size();
+        int rc = intern_materials(s, packed, count);
+        if (rc == MPM_OK && (s->mats.size() != before || s->d_mats == nullptr)) rc = upload_materials(s);
+        if (rc != MPM_OK) return rc;
+    }
+    for (uint32_t first = 0; first < count; first += s->slab_records) {
+        const uint32_t n = std::min(count - first, s->slab_records);
+        if (!one_slab)
+            CUDA_TRY(s->stage->copy_in(s->stream, records, packed + (size_t)first * MPM_PARTICLE_WORDS,
+                                       (size_t)n * record));
+        k_unpack_records<<<blocks_for(n, RECORD_THREADS), RECORD_THREADS, 0, s->stream>>>(
+            records, n, s->d_mats, (uint32_t)s->mats.size(), s->buf[target], s->bonded, s->slot_of[target],
+            slot_base + first, orig_base + first);
+        CUDA_TRY(cudaGetLastError());
+    }
     return MPM_OK;
 }
 
@@ -828,9 +833,10 @@ void free_solver(mpm_solver *s)
                     s->tmp, s->perm, s->cell_count, s->cell_start, s->block_sums, s->p2g_solid, s->p2g_water,
                     s->p2g_oil, s->g_solid, s->g_water, s->g_oil, s->fixed, s->tile_stamp, s->d_active,
                     s->tile_count, s->tile_range, s->scene_chunk, s->active_tiles, s->part, s->tile_info,
-                    s->rec_state, s->rec_affine, s->rec_mom, s->rec_cell, s->field, s->body_starts,
+                    s->field, s->body_starts,
                     s->slot_of[0], s->slot_of[1], s->track_flag, s->tracked, s->pair_cache, s->contact_count,
-                    s->body_vel, s->bonds, s->topology, s->endpoints, s->surface_acc, s->surface_field};
+                    s->body_vel, s->bonds, s->topology, s->endpoints, s->surface_acc, s->surface_field,
+                    s->slab};
     for (void *p : ptrs)
         if (p) cudaFree(p);
     for (int b = 0; b < 2; ++b) {
@@ -841,6 +847,7 @@ void free_solver(mpm_solver *s)
     }
     if (s->h_params) cudaFreeHost(s->h_params);
     if (s->h_readback) cudaFreeHost(s->h_readback);
+    if (s->stage) s->stage->release();
     if (s->params_copied) cudaEventDestroy(s->params_copied);
     if (s->batch_start) cudaEventDestroy(s->batch_start);
     if (s->batch_stop) cudaEventDestroy(s->batch_stop);
@@ -930,6 +937,8 @@ int create_impl(const mpm_config *configs, uint32_t n_scenes, const uint32_t *co
 
     mpm_solver *s = new mpm_solver();
     s->device = c.device;
+    s->stage = &RecordStage::of(c.device);
+    s->stage->retain();
     s->cfg = c;
     s->n = count;
     s->allocated = count;
@@ -996,6 +1005,7 @@ int create_impl(const mpm_config *configs, uint32_t n_scenes, const uint32_t *co
     cudaEventRecord(s->params_copied, s->stream);
 
     const size_t cap = s->capacity;
+    const bool gather = c.p2g_mode == MPM_P2G_GATHER;
     ALLOC(s->d_params, n_scenes);
     ALLOC(s->dyn, (size_t)n_scenes * SCENE_WORDS);
     ALLOC(s->work, WORK_WORDS);
@@ -1019,6 +1029,9 @@ int create_impl(const mpm_config *configs, uint32_t n_scenes, const uint32_t *co
     ALLOC(s->ranks, cap);
     ALLOC(s->tmp, cap);
     ALLOC(s->perm, cap);
+    s->slab_records = (uint32_t)std::min<size_t>(cap, RECORD_SLAB);
+    ALLOC(s->slab, std::max(gather ? cap * P2G_RECORD_BYTES : 0,
+                            s->slab_records * (MPM_PARTICLE_WORDS + 1) * sizeof(float)));
     ALLOC(s->cell_count, s->cell_pad);
     ALLOC(s->cell_start, (size_t)s->cell_pad + 1);
     ALLOC(s->block_sums, (size_t)s->n_chunks + 1);
@@ -1061,10 +1074,10 @@ int create_impl(const mpm_config *configs, uint32_t n_scenes, const uint32_t *co
         ALLOC(s->active_tiles, n_tiles);
         ALLOC(s->part, n_tiles * ACC_WORDS * RING_NODES);
         ALLOC(s->tile_info, n_tiles);
-        ALLOC(s->rec_state, cap);
-        ALLOC(s->rec_affine, cap);
-        ALLOC(s->rec_mom, cap);
-        ALLOC(s->rec_cell, cap);
+        s->rec_state = reinterpret_cast<float4 *>(s->slab);
+        s->rec_affine = s->rec_state + cap;
+        s->rec_mom = reinterpret_cast<float2 *>(s->rec_affine + cap);
+        s->rec_cell = reinterpret_cast<uint32_t *>(s->rec_mom + cap);
         if (cudaMemsetAsync(s->tile_info, 0xff, n_tiles * sizeof(uint2), s->stream) != cudaSuccess ||
             cudaMemsetAsync(s->tile_count, 0, n_tiles * sizeof(uint32_t), s->stream) != cudaSuccess)
             return fail(set_error(MPM_ERR_CUDA, "cudaMemset failed"));
@@ -1377,6 +1390,16 @@ namespace {
 // (see capture_batch); longer ones launch graphs of 2^k substeps.
 constexpr uint32_t MAX_BATCH_GRAPH_STEPS = 16;
 
+// Queues the compact readback (counters and status words) to pinned memory.
+cudaError_t copy_readback(mpm_solver *s)
+{
+    const cudaError_t e = cudaMemcpyAsync(s->h_readback, s->d_counters + COUNTER_PROGRESS, 2 * sizeof(uint32_t),
+                                          cudaMemcpyDeviceToHost, s->stream);
+    return e != cudaSuccess ? e
+                            : cudaMemcpyAsync(s->h_readback + 2, s->d_status, 8 * sizeof(uint32_t),
+                                              cudaMemcpyDeviceToHost, s->stream);
+}
+
 // The whole batch on the stream being captured: the parameter copy from
 // pinned memory, the batch events, the prologue, the substeps, the epilogue
 // and the compact readback (counters and status words) to pinned memory.
@@ -1398,12 +1421,7 @@ cudaError_t capture_batch(mpm_solver *s, uint32_t step_count, int parity, bool g
     enqueue_end_batch(s, p, step_count, guarded);
     e = cudaGetLastError();
     if (e == cudaSuccess) e = cudaEventRecordWithFlags(s->batch_stop, s->stream, cudaEventRecordExternal);
-    if (e == cudaSuccess)
-        e = cudaMemcpyAsync(s->h_readback, s->d_counters + COUNTER_PROGRESS, 2 * sizeof(uint32_t),
-                            cudaMemcpyDeviceToHost, s->stream);
-    if (e == cudaSuccess)
-        e = cudaMemcpyAsync(s->h_readback + 2, s->d_status, 8 * sizeof(uint32_t), cudaMemcpyDeviceToHost, s->stream);
-    return e;
+    return e == cudaSuccess ? copy_readback(s) : e;
 }
 
 int get_batch_graph(mpm_solver *s, uint32_t step_count, int parity, bool guarded, cudaGraphExec_t *out)
@@ -1475,6 +1493,8 @@ int run_batch(mpm_solver *s, uint32_t step_count, bool guarded)
     }
     CUDA_TRY(cudaEventRecord(s->batch_stop, s->stream));
     s->batch_timed = true;
+    CUDA_TRY(copy_readback(s));
+    s->readback_ready = true;
     return MPM_OK;
 }
 
@@ -1789,12 +1809,7 @@ int mpm_read_compact(mpm_solver *s, float *maximum_speed, uint32_t *completed, u
     g_last_error.clear();
     if (!s) return set_error(MPM_ERR_INVALID_ARGUMENT, "solver must not be NULL");
     CUDA_TRY(cudaSetDevice(s->device));
-    if (!s->readback_ready) {
-        CUDA_TRY(cudaMemcpyAsync(s->h_readback, s->d_counters + COUNTER_PROGRESS, 2 * sizeof(uint32_t),
-                                 cudaMemcpyDeviceToHost, s->stream));
-        CUDA_TRY(cudaMemcpyAsync(s->h_readback + 2, s->d_status, 8 * sizeof(uint32_t), cudaMemcpyDeviceToHost,
-                                 s->stream));
-    }
+    if (!s->readback_ready) CUDA_TRY(copy_readback(s));
     CUDA_TRY(cudaStreamSynchronize(s->stream));
     if (s->batch_timed && !s->batch_ms_known) {
         // the batch has ended: its time is read now, for mpm_last_batch_device_ms
@@ -1837,54 +1852,62 @@ int mpm_read_particles(mpm_solver *s, const uint32_t *indices, uint32_t count, f
     if (!indices && count != total) return set_error(MPM_ERR_INVALID_ARGUMENT, "count must equal the particle count");
     for (uint32_t k = 0; indices && k < count; ++k)
         if (indices[k] >= total) return set_error(MPM_ERR_INVALID_ARGUMENT, "particleIndices must identify active GPU particles.");
+    if (count == 0) return MPM_OK;
     CUDA_TRY(cudaSetDevice(s->device));
-    const uint32_t n = s->n;
-    HostState h;
-    int rc = download_state(s, h);
-    if (rc != MPM_OK) return rc;
-    std::vector<uint32_t> bonded(total), obj(total), slot_of(total, 0xffffffffu);
-    if (total > 0) {
-        CUDA_TRY(cudaMemcpyAsync(bonded.data(), s->bonded, total * sizeof(uint32_t), cudaMemcpyDeviceToHost, s->stream));
-        CUDA_TRY(cudaMemcpyAsync(obj.data(), s->obj, total * sizeof(uint32_t), cudaMemcpyDeviceToHost, s->stream));
-        CUDA_TRY(cudaStreamSynchronize(s->stream));
+    const size_t record = MPM_PARTICLE_WORDS * sizeof(float);
+    const size_t width = record + (object_ids_out ? sizeof(uint32_t) : 0);
+    const uint32_t most = std::min(count, s->slab_records);
+    uint32_t *const d_flags = s->h_readback + READBACK_FLAGS;
+    // [0] a slot names no particle, [1] requested indices without a slot
+    volatile uint32_t *const flags = d_flags;
+    flags[0] = flags[1] = 0u;
+    const bool all = !indices && s->n == total && most == count;  // every index has a slot
+    if (!all) {
+        if (s->n > 0)
+            k_record_slots<<<blocks_for(s->n, RECORD_THREADS), RECORD_THREADS, 0, s->stream>>>(
+                s->buf[s->cur].orig, s->n, total, s->tmp, d_flags);
     }
-    for (uint32_t d = 0; d < n; ++d) {
-        if (h.orig[d] >= total) return set_error(MPM_ERR_CUDA, "corrupt particle slot map");
-        slot_of[h.orig[d]] = d;
-    }
-    for (uint32_t k = 0; k < count; ++k) {
-        const uint32_t i = indices ? indices[k] : k;
-        const uint32_t d = slot_of[i];
-        float *w = packed_out + (size_t)k * MPM_PARTICLE_WORDS;
-        if (object_ids_out) object_ids_out[k] = obj[i];
-        if (d == 0xffffffffu) {
-            // removed by an outlet: its last state, material model 0xffffffff
-            // (MODEL_REMOVED, shaders.ts:195)
-            if (i >= s->removed.size() || !s->removed[i]) return set_error(MPM_ERR_CUDA, "corrupt particle slot map");
-            std::memcpy(w, s->removed_words.data() + (size_t)i * MPM_PARTICLE_WORDS, MPM_PARTICLE_WORDS * sizeof(float));
-            continue;
+    // what fits one chunk the kernel writes straight to pinned memory, the rest
+    // goes through the device slab
+    void *lent = s->stage->lend((size_t)count * width);
+    const ReturnChunk give_back{s, lent != nullptr};
+    unsigned char *const out = lent ? static_cast<unsigned char *>(lent) : s->slab;
+    for (uint32_t first = 0; first < count; first += most) {
+        const uint32_t n = std::min(count - first, most);
+        const unsigned ctas = blocks_for(n, RECORD_THREADS);
+        float *const records = reinterpret_cast<float *>(out);
+        uint32_t *const ids = object_ids_out ? reinterpret_cast<uint32_t *>(out + (size_t)n * record) : nullptr;
+        if (all) {
+            k_pack_all_records<<<ctas, RECORD_THREADS, 0, s->stream>>>(s->buf[s->cur], n, s->d_mats, s->bonded, s->obj,
+                                                                       records, ids, d_flags);
+        } else {
+            if (indices)
+                CUDA_TRY(cudaMemcpyAsync(s->keys, indices + first, n * sizeof(uint32_t), cudaMemcpyHostToDevice,
+                                         s->stream));
+            k_pack_records<<<ctas, RECORD_THREADS, 0, s->stream>>>(s->buf[s->cur], s->n, s->d_mats, s->bonded, s->obj,
+                                                                   s->tmp, indices ? s->keys : nullptr,
+                                                                   first, n, records, ids, d_flags + 1);
         }
-        const Material &m = s->mats[h.mat[d]];
-        w[0] = h.pos[d].x;
-        w[1] = h.pos[d].y;
-        w[2] = h.vel[d].x;
-        w[3] = h.vel[d].y;
-        w[4] = h.C[d].x;
-        w[5] = h.C[d].y;
-        w[6] = h.C[d].z;
-        w[7] = h.C[d].w;
-        w[8] = h.F[d].x;
-        w[9] = h.F[d].y;
-        w[10] = h.F[d].z;
-        w[11] = h.F[d].w;
-        w[12] = h.pvol[d];
-        w[13] = u2f(m.model);
-        w[14] = m.lambda;
-        w[15] = m.mu;
-        w[16] = m.density;
-        w[17] = h.vol[d];
-        w[18] = m.model == MODEL_NEO_HOOKEAN ? h.damage[d] : m.param;
-        w[19] = u2f(bonded[i]);
+        CUDA_TRY(cudaGetLastError());
+        float *const host_records = packed_out + (size_t)first * MPM_PARTICLE_WORDS;
+        if (lent) {
+            CUDA_TRY(cudaStreamSynchronize(s->stream));
+            std::memcpy(host_records, out, (size_t)n * record);
+            if (ids) std::memcpy(object_ids_out + first, out + (size_t)n * record, (size_t)n * sizeof(uint32_t));
+        } else {
+            CUDA_TRY(s->stage->copy_out(s->stream, out, (size_t)n * width, host_records, (size_t)n * record,
+                                       object_ids_out ? object_ids_out + first : nullptr));
+        }
+    }
+    if (flags[0] != 0u) return set_error(MPM_ERR_CUDA, "corrupt particle slot map");
+    for (uint32_t k = 0; flags[1] != 0u && k < count; ++k) {
+        float *w = packed_out + (size_t)k * MPM_PARTICLE_WORDS;
+        if (f2u(w[13]) != 0xffffffffu) continue;
+        // removed by an outlet: its last state, material model 0xffffffff
+        // (MODEL_REMOVED, shaders.ts:195)
+        const uint32_t i = indices ? indices[k] : k;
+        if (i >= s->removed.size() || !s->removed[i]) return set_error(MPM_ERR_CUDA, "corrupt particle slot map");
+        std::memcpy(w, s->removed_words.data() + (size_t)i * MPM_PARTICLE_WORDS, record);
     }
     return MPM_OK;
 }
