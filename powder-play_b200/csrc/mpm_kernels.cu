@@ -1015,8 +1015,10 @@ struct Stage {
     float2 momentum[CAP];  // m v
     uint32_t orig[CAP];    // original index; after the count pass channel << 30 | original index
     uint32_t cell[CAP];    // local cell | channel << 8 | REC_FAILED
-    uint16_t order[CAP];   // arrival rank within the cell, then rank by (channel, original index)
-    uint16_t sorted[CAP];  // staged indices grouped by cell
+    uint32_t key[CAP];     // the sort keys grouped by cell, in arrival order
+    uint16_t grouped[CAP]; // staged indices grouped by cell, in arrival order
+    uint16_t sorted[CAP];  // arrival rank within the cell; then the staged indices grouped by cell, by
+                           // (channel, original index) within it
     uint32_t count[TILE_CELLS];
     uint32_t start[TILE_CELLS + 1];
     float acc[ACC_WORDS][RING_NODES];
@@ -1027,48 +1029,6 @@ struct Stage {
     int failed;
     uint32_t item;  // the tile this group claimed (several scenes)
 };
-
-// A P2G tile is taken by a group of TILE_CELLS threads (one per cell of the
-// tile in the count and scan passes): the whole CTA of k_p2g_gather, or one
-// of the GROUPS halves of a k_substep CTA, which then synchronise on named
-// barriers 1 and 2 (barrier 0 stays the CTA's).
-template <int GROUPS>
-__device__ __forceinline__ uint32_t p2g_group() { return GROUPS == 1 ? 0u : threadIdx.x / TILE_CELLS; }
-
-template <int GROUPS>
-__device__ __forceinline__ void group_sync()
-{
-    if constexpr (GROUPS == 1) {
-        __syncthreads();
-    } else {
-        // barrier ids as immediates (the group is uniform per warp)
-        if (p2g_group<GROUPS>() == 0u)
-            asm volatile("bar.sync 1, %0;" ::"n"(TILE_CELLS) : "memory");
-        else
-            asm volatile("bar.sync 2, %0;" ::"n"(TILE_CELLS) : "memory");
-    }
-}
-
-template <int GROUPS>
-__device__ __forceinline__ uint32_t group_sync_count(bool pred)
-{
-    if constexpr (GROUPS == 1) {
-        return (uint32_t)__syncthreads_count(pred);
-    } else {
-        uint32_t r;
-        if (p2g_group<GROUPS>() == 0u)
-            asm volatile("{\n .reg .pred p;\n setp.ne.u32 p, %1, 0;\n bar.red.popc.u32 %0, 1, %2, p;\n}\n"
-                         : "=r"(r)
-                         : "r"(pred ? 1u : 0u), "n"(TILE_CELLS)
-                         : "memory");
-        else
-            asm volatile("{\n .reg .pred p;\n setp.ne.u32 p, %1, 0;\n bar.red.popc.u32 %0, 2, %2, p;\n}\n"
-                         : "=r"(r)
-                         : "r"(pred ? 1u : 0u), "n"(TILE_CELLS)
-                         : "memory");
-        return r;
-    }
-}
 
 // First sorted entry of channel >= ch in the cell's entries [lo, hi) (they
 // are ordered by channel, then original index).
@@ -1083,12 +1043,6 @@ __device__ __forceinline__ uint32_t channel_start(const Stage<CAP> &sm, uint32_t
             hi = mid;
     }
     return lo;
-}
-
-template <int CAP>
-__device__ __forceinline__ uint32_t sort_key(const Stage<CAP> &sm, uint32_t k)
-{
-    return sm.orig[k];  // channel << 30 | original index, set by p2g_chunk's count pass
 }
 
 // Exclusive scan of the 128 cell counts by the group's first warp (4 cells
@@ -1118,6 +1072,57 @@ __device__ __forceinline__ void scan_cell_counts(uint32_t lane, const uint32_t *
     }
 }
 
+// The P2G sums of one cell's particles at the stencil nodes of one thread: all
+// nine (ROLES 1) or, row-major, the first five or the other four (ROLES 2).
+template <int ROLES>
+struct NodeSums {
+    static constexpr int NODES = ROLES == 1 ? 9 : 5;
+    float m[NODES], px[NODES], py[NODES], vl[NODES];
+};
+
+// Adds the sorted entries from, from + share, ... below `to` at the stencil
+// nodes O0 .. O1 - 1 to q, then the partial sums of a cell's `share` threads
+// pairwise (lane + off into lane).
+template <int O0, int O1, int CAP, int ROLES>
+__device__ __forceinline__ void sum_nodes(const Stage<CAP> &sm, uint32_t from, uint32_t to, uint32_t share, float dx,
+                                          NodeSums<ROLES> &q)
+{
+    for (uint32_t j = from; j < to; j += share) {
+        const uint32_t k = sm.sorted[j];
+        const float4 s = sm.state[k];
+        const float4 A = sm.affine[k];
+        const float2 mv = sm.momentum[k];
+        float wx[3], wy[3], dpx[3], dpy[3];
+#pragma unroll
+        for (int t = 0; t < 3; ++t) {
+            wx[t] = quad_weight(s.x, t);
+            wy[t] = quad_weight(s.y, t);
+            dpx[t] = ((float)t - s.x) * dx;
+            dpy[t] = ((float)t - s.y) * dx;
+        }
+#pragma unroll
+        for (int o = O0; o < O1; ++o) {
+            const int ox = o % 3, oy = o / 3;
+            const float w = wx[ox] * wy[oy];
+            const float mx = mv.x + A.x * dpx[ox] + A.y * dpy[oy];
+            const float my = mv.y + A.z * dpx[ox] + A.w * dpy[oy];
+            q.m[o - O0] += w * s.z;
+            q.px[o - O0] += w * mx;
+            q.py[o - O0] += w * my;
+            q.vl[o - O0] += w * s.w;
+        }
+    }
+    for (uint32_t off = share / 2u; off > 0u; off /= 2u) {
+#pragma unroll
+        for (int i = 0; i < O1 - O0; ++i) {
+            q.m[i] += __shfl_down_sync(0xffffffffu, q.m[i], off, (int)share);
+            q.px[i] += __shfl_down_sync(0xffffffffu, q.px[i], off, (int)share);
+            q.py[i] += __shfl_down_sync(0xffffffffu, q.py[i], off, (int)share);
+            q.vl[i] += __shfl_down_sync(0xffffffffu, q.vl[i], off, (int)share);
+        }
+    }
+}
+
 // Stages the particles of the slots src[i0 .. i1) with asynchronous copies
 // and prepares each of them in shared memory (REC: stages the records G2P
 // wrote), raises the status of failed preparations and groups the entries by
@@ -1127,30 +1132,31 @@ __device__ __forceinline__ void scan_cell_counts(uint32_t lane, const uint32_t *
 // in nine phases, one stencil offset per phase (no two cells of a phase share
 // a node), so every sum has a fixed order.  Returns false once a particle
 // failed.
-template <int CAP, int GROUPS, bool LIQ, bool REC>
+template <int CAP, int ROLES, bool LIQ, bool REC>
 __device__ __forceinline__ bool p2g_chunk(const Ctx &c, Stage<CAP> &sm, const uint32_t *src, uint32_t i0, uint32_t i1)
 {
+    constexpr uint32_t THREADS = ROLES * TILE_CELLS;
     const StepParams &P = *c.P;
-    const uint32_t me = threadIdx.x % TILE_CELLS;  // this thread's cell
-    sm.count[me] = 0u;
-    group_sync<GROUPS>();
+    const uint32_t me = threadIdx.x;
+    if (me < (uint32_t)TILE_CELLS) sm.count[me] = 0u;  // the first threads: one per cell
+    __syncthreads();
     const uint32_t n = i1 - i0;
     // Up to the cell counts every thread works on the entries it copies in
-    // itself (k = me, me + TILE_CELLS, ...), which its own cp.async wait makes
+    // itself (k = me, me + THREADS, ...), which its own cp.async wait makes
     // visible to it, so no group barrier is needed before the counts are read.
     uint32_t mask = 0;
     // the entry's arrival rank within its cell; from here on its word holds
     // its sort key: channel in the top two bits over the original index
     // (below 2^30: far more particles than the device memory holds)
     auto count_entry = [&](uint32_t k, uint32_t cell) {
-        sm.order[k] = (uint16_t)atomicAdd(&sm.count[cell & 0xffu], 1u);
+        sm.sorted[k] = (uint16_t)atomicAdd(&sm.count[cell & 0xffu], 1u);
         mask |= 1u << ((cell >> 8) & 3u);
         sm.orig[k] |= ((cell >> 8) & 3u) << 30;
     };
     if constexpr (REC) {
         // the records variant: the P2G records the previous G2P (or the
         // batch prologue) wrote
-        for (uint32_t i = i0 + me; i < i1; i += TILE_CELLS) {
+        for (uint32_t i = i0 + me; i < i1; i += THREADS) {
             const uint32_t s = src[i];
             const uint32_t k = i - i0;
             cp_async<16>(&sm.state[k], &c.rec_state[s]);
@@ -1160,7 +1166,7 @@ __device__ __forceinline__ bool p2g_chunk(const Ctx &c, Stage<CAP> &sm, const ui
             cp_async<4>(&sm.cell[k], &c.rec_cell[s]);
         }
         cp_async_wait_all();
-        for (uint32_t k = me; k < n; k += TILE_CELLS) {
+        for (uint32_t k = me; k < n; k += THREADS) {
             const uint32_t cell = sm.cell[k];
             if (cell & REC_FAILED) {  // the record carries prepareParticle's flags
                 const float4 f = sm.state[k];
@@ -1178,12 +1184,12 @@ __device__ __forceinline__ bool p2g_chunk(const Ctx &c, Stage<CAP> &sm, const ui
         // into the slots their results replace (state, affine, momentum, cell);
         // position, volume (and damage and plastic volume for the general
         // models) loaded into this thread's registers while the copies fly
-        constexpr int PER = (CAP + TILE_CELLS - 1) / TILE_CELLS;  // entries per thread
+        constexpr int PER = (CAP + THREADS - 1) / THREADS;  // entries per thread
         float2 pos[PER];
         float vol[PER], dmg[PER], pvl[PER];
 #pragma unroll
         for (int u = 0; u < PER; ++u) {
-            const uint32_t i = i0 + me + (uint32_t)u * TILE_CELLS;
+            const uint32_t i = i0 + me + (uint32_t)u * THREADS;
             if (i < i1) {
                 const uint32_t s = src[i];
                 const uint32_t k = i - i0;
@@ -1206,7 +1212,7 @@ __device__ __forceinline__ bool p2g_chunk(const Ctx &c, Stage<CAP> &sm, const ui
         // local cell | channel << 8 (| REC_FAILED after raising its status)
 #pragma unroll
         for (int u = 0; u < PER; ++u) {
-            const uint32_t k = me + (uint32_t)u * TILE_CELLS;
+            const uint32_t k = me + (uint32_t)u * THREADS;
             if (k < n) {
                 const Material m = c.mats[sm.cell[k]];
                 const float4 F = sm.state[k], C = sm.affine[k];
@@ -1246,120 +1252,89 @@ __device__ __forceinline__ bool p2g_chunk(const Ctx &c, Stage<CAP> &sm, const ui
         }
     }
     if (mask) atomicOr(&sm.mask, mask);
-    group_sync<GROUPS>();
+    __syncthreads();
     if (sm.failed) return false;
     if (me < 32) scan_cell_counts(me, sm.count, sm.start, nullptr);
-    group_sync<GROUPS>();
-    for (uint32_t k = me; k < n; k += TILE_CELLS) sm.sorted[sm.start[sm.cell[k] & 0xffu] + sm.order[k]] = (uint16_t)k;
-    group_sync<GROUPS>();
+    __syncthreads();
+    for (uint32_t k = me; k < n; k += THREADS) {
+        const uint32_t p = sm.start[sm.cell[k] & 0xffu] + sm.sorted[k];
+        sm.grouped[p] = (uint16_t)k;
+        sm.key[p] = sm.orig[k];
+    }
+    __syncthreads();
     // order each cell's entries by (channel, original index): every entry
     // counts the entries of its cell with a smaller key (keys are distinct),
     // so crowded cells spread over all threads
-    for (uint32_t k = me; k < n; k += TILE_CELLS) {
-        const uint32_t cell = sm.cell[k] & 0xffu, key = sort_key(sm, k);
-        uint32_t rank = 0;
-        for (uint32_t j = sm.start[cell]; j < sm.start[cell + 1]; ++j) rank += sort_key(sm, sm.sorted[j]) < key;
-        sm.order[k] = (uint16_t)rank;
+    for (uint32_t p = me; p < n; p += THREADS) {
+        const uint32_t k = sm.grouped[p], key = sm.key[p], cell = sm.cell[k] & 0xffu;
+        const uint32_t lo = sm.start[cell], hi = sm.start[cell + 1];
+        uint32_t at = lo;
+        for (uint32_t j = lo; j < hi; ++j) at += sm.key[j] < key;
+        sm.sorted[at] = (uint16_t)k;
     }
-    group_sync<GROUPS>();
-    for (uint32_t k = me; k < n; k += TILE_CELLS) sm.sorted[sm.start[sm.cell[k] & 0xffu] + sm.order[k]] = (uint16_t)k;
-    group_sync<GROUPS>();
+    __syncthreads();
     // the cells holding entries, compacted; each gets a group of `share`
     // consecutive threads of one warp (a power of two up to 32, so that the
     // groups fill the 128 threads): a crowded chunk of few cells spreads each
     // cell's particles over its group, which adds their sums in a fixed tree
     // order (with more than 64 such cells every thread takes its own cell)
-    const bool has = sm.start[me + 1] > sm.start[me];
-    const uint32_t n_cells = group_sync_count<GROUPS>(has);
+    const uint32_t seat = me % TILE_CELLS;  // this thread's place among the threads of its role
+    const uint32_t role = ROLES == 1 ? 0u : me / TILE_CELLS;  // which of the stencil's nodes it sums
+    const bool has = role == 0u && sm.start[seat + 1] > sm.start[seat];
+    const uint32_t n_cells = (uint32_t)__syncthreads_count(has);
     uint32_t share = 1;
     while (share < 32u && n_cells * share * 2u <= (uint32_t)TILE_CELLS) share *= 2u;
     if (share > 1u) {
         const unsigned ballot = __ballot_sync(0xffffffffu, has);
         const uint32_t lane = me & 31u, warp = me >> 5;
-        if (lane == 0u) sm.warp_active[warp] = __popc(ballot);
-        group_sync<GROUPS>();
-        uint32_t before = 0;
-        for (uint32_t w = 0; w < warp; ++w) before += sm.warp_active[w];
-        if (has) sm.active[before + __popc(ballot & ((1u << lane) - 1u))] = (uint8_t)me;
-        group_sync<GROUPS>();
+        if (lane == 0u && role == 0u) sm.warp_active[warp] = __popc(ballot);
+        __syncthreads();
+        if (has) {
+            uint32_t before = 0;
+            for (uint32_t w = 0; w < warp; ++w) before += sm.warp_active[w];
+            sm.active[before + __popc(ballot & ((1u << lane) - 1u))] = (uint8_t)seat;
+        }
+        __syncthreads();
     }
-    const uint32_t group = me / share, part = me % share;
+    const uint32_t group = seat / share, part = seat % share;
     const bool mine = share == 1u || group < n_cells;
-    const uint32_t cell = share == 1u ? me : (mine ? sm.active[group] : 0u);
+    const uint32_t cell = share == 1u ? seat : (mine ? sm.active[group] : 0u);
     const uint32_t lo = mine ? sm.start[cell] : 0u, hi = mine ? sm.start[cell + 1] : 0u;
-    const int cx = (int)(cell % TILE_X), cy = (int)(cell / TILE_X);
+    const uint32_t ring = (cell / TILE_X) * RING_X + cell % TILE_X;  // the cell's first ring node
     const float dx = P.dx;
     const uint32_t tile_mask = sm.mask;
     uint32_t lo_ch = lo;
 #pragma unroll 1
     for (uint32_t ch = 0; ch < 3u; ++ch) {
         if (!(tile_mask & (1u << ch))) continue;
-        float m[9], px[9], py[9], vl[9];
+        NodeSums<ROLES> q;
+        constexpr int NODES = NodeSums<ROLES>::NODES;
 #pragma unroll
-        for (int o = 0; o < 9; ++o) m[o] = px[o] = py[o] = vl[o] = 0.f;
+        for (int o = 0; o < NODES; ++o) q.m[o] = q.px[o] = q.py[o] = q.vl[o] = 0.f;
         // this channel's entries of the cell: [a, b)
         const uint32_t a = lo_ch;
-        const uint32_t b = ch == 2u ? hi : channel_start(sm, a, hi, ch + 1u);
+        const uint32_t b = (tile_mask >> (ch + 1u)) == 0u ? hi : channel_start(sm, a, hi, ch + 1u);
         lo_ch = b;
-        for (uint32_t j = a + part; j < b; j += share) {
-            const uint32_t k = sm.sorted[j];
-            const float4 q = sm.state[k];
-            const float4 A = sm.affine[k];
-            const float2 mv = sm.momentum[k];
-            float wx[3], wy[3], dpx[3], dpy[3];
-#pragma unroll
-            for (int t = 0; t < 3; ++t) {
-                wx[t] = quad_weight(q.x, t);
-                wy[t] = quad_weight(q.y, t);
-                dpx[t] = ((float)t - q.x) * dx;
-                dpy[t] = ((float)t - q.y) * dx;
-            }
-#pragma unroll
-            for (int oy = 0; oy < 3; ++oy) {
-#pragma unroll
-                for (int ox = 0; ox < 3; ++ox) {
-                    const int o = oy * 3 + ox;
-                    const float w = wx[ox] * wy[oy];
-                    const float mx = mv.x + A.x * dpx[ox] + A.y * dpy[oy];
-                    const float my = mv.y + A.z * dpx[ox] + A.w * dpy[oy];
-                    m[o] += w * q.z;
-                    px[o] += w * mx;
-                    py[o] += w * my;
-                    vl[o] += w * q.w;
-                }
-            }
-        }
-        if (share > 1u) {
-            // the group's partial sums, added pairwise (lane + off into lane)
-            for (uint32_t off = share / 2u; off > 0u; off /= 2u) {
-#pragma unroll
-                for (int o = 0; o < 9; ++o) {
-                    m[o] += __shfl_down_sync(0xffffffffu, m[o], off, (int)share);
-                    px[o] += __shfl_down_sync(0xffffffffu, px[o], off, (int)share);
-                    py[o] += __shfl_down_sync(0xffffffffu, py[o], off, (int)share);
-                    vl[o] += __shfl_down_sync(0xffffffffu, vl[o], off, (int)share);
-                }
-            }
-        }
+        if (ROLES == 1 || role == 0u)
+            sum_nodes<0, NODES>(sm, a + part, b, share, dx, q);
+        else
+            sum_nodes<ROLES == 1 ? 0 : NODES, 9>(sm, a + part, b, share, dx, q);
         const bool adds = mine && part == 0u;
         const int word = ch == 0u ? 0 : (ch == 1u ? 3 : 7);
 #pragma unroll
-        for (int oy = 0; oy < 3; ++oy) {
-#pragma unroll
-            for (int ox = 0; ox < 3; ++ox) {
-                const int o = oy * 3 + ox;
-                group_sync<GROUPS>();  // the previous phase's adds are done
-                if (adds) {
-                    const int r = (cy + oy) * RING_X + cx + ox;
-                    sm.acc[word][r] += m[o];
-                    sm.acc[word + 1][r] += px[o];
-                    sm.acc[word + 2][r] += py[o];
-                    if (ch != 0u) sm.acc[word + 3][r] += vl[o];
-                }
+        for (int o = 0; o < 9; ++o) {
+            __syncthreads();  // the previous phase's adds are done
+            if (adds && role == (uint32_t)(o / NODES)) {
+                const int i = o % NODES;
+                const uint32_t r = ring + (uint32_t)((o / 3) * RING_X + o % 3);
+                sm.acc[word][r] += q.m[i];
+                sm.acc[word + 1][r] += q.px[i];
+                sm.acc[word + 2][r] += q.py[i];
+                if (ch != 0u) sm.acc[word + 3][r] += q.vl[i];
             }
         }
     }
-    group_sync<GROUPS>();
+    __syncthreads();
     return true;
 }
 
@@ -1373,41 +1348,39 @@ __device__ __forceinline__ bool p2g_chunk(const Ctx &c, Stage<CAP> &sm, const ui
 // consecutive whole cells (a cell holding more than CAP particles in chunks
 // of the bucket, whose order then decides the rounding of its sums).  The
 // sums go to the tile's own ring record; the G2P adds the up to four
-// records that cover a node.  The GROUPS groups of a CTA take interleaved
-// tiles of the list, each with its own stage.
-template <bool SCENES, int CAP, int GROUPS, bool LIQ, bool REC>
-__device__ __forceinline__ void p2g_tiles(const Ctx &c0, Stage<CAP> *stages)
+// records that cover a node.
+template <bool SCENES, int CAP, int ROLES, bool LIQ, bool REC>
+__device__ __forceinline__ void p2g_tiles(const Ctx &c0, Stage<CAP> &sm)
 {
-    const uint32_t g = p2g_group<GROUPS>();
-    const uint32_t me = threadIdx.x % TILE_CELLS;
-    Stage<CAP> &sm = stages[g];
+    constexpr uint32_t THREADS = ROLES * TILE_CELLS;
+    const uint32_t me = threadIdx.x;
     const uint32_t n_active = listed_count(c0), n_heavy = heavy_count(c0);
-    // several scenes: each group claims its next tile (the heavy ones are
+    // several scenes: each CTA claims its next tile (the heavy ones are
     // listed first), which evens out tiles of very different sizes; one scene
     // (tiles of similar size): a fixed stride
     auto next = [&](uint32_t prev) -> uint32_t {
         if constexpr (SCENES) {
-            group_sync<GROUPS>();  // the readers of the previous claim are done
+            __syncthreads();  // the readers of the previous claim are done
             if (me == 0) sm.item = atomicAdd(c0.work + WORK_CLAIM, 1u);
-            group_sync<GROUPS>();
+            __syncthreads();
             return sm.item;
         } else {
-            return prev + gridDim.x * GROUPS;
+            return prev + gridDim.x;
         }
     };
-    for (uint32_t item = SCENES ? next(0u) : blockIdx.x * GROUPS + g; item < n_active; item = next(item)) {
+    for (uint32_t item = SCENES ? next(0u) : blockIdx.x; item < n_active; item = next(item)) {
         const uint32_t tile = __ldcg(listed_tile(c0, item, n_heavy));
         const Ctx c = tile_ctx<SCENES>(c0, tile);
         const uint32_t stamp = __ldcg(c.counters + COUNTER_STAMP);
         const uint2 range = __ldcg(c.tile_range + tile);
         const uint32_t begin = range.x, n_tile = range.y;
-        group_sync<GROUPS>();  // the previous tile's readers of sm are done
-        for (int k = me; k < ACC_WORDS * RING_NODES; k += TILE_CELLS) (&sm.acc[0][0])[k] = 0.f;
+        __syncthreads();  // the previous tile's readers of sm are done
+        for (int k = me; k < ACC_WORDS * RING_NODES; k += THREADS) (&sm.acc[0][0])[k] = 0.f;
         if (me == 0) {
-            sm.failed = *(volatile uint32_t *)c.status != 0u ? 1 : 0;  // one read for the whole group
+            sm.failed = *(volatile uint32_t *)c.status != 0u ? 1 : 0;  // one read for the whole CTA
             sm.mask = 0u;
         }
-        group_sync<GROUPS>();
+        __syncthreads();
         if (sm.failed) continue;  // the scene's substep is rolled back
         // a tile above one stage: its entries are first ordered by cell into
         // the scratch list tmp[begin .. begin + n_tile) (arrival order within
@@ -1416,34 +1389,32 @@ __device__ __forceinline__ void p2g_tiles(const Ctx &c0, Stage<CAP> *stages)
         // its list, whose arrival order then decides the rounding
         const uint32_t *src = c.perm + begin;
         if (n_tile > (uint32_t)CAP) {
-            sm.count[me] = 0u;  // one thread per cell
-            group_sync<GROUPS>();
-            for (uint32_t i = me; i < n_tile; i += 4 * TILE_CELLS) {
+            if (me < (uint32_t)TILE_CELLS) sm.count[me] = 0u;
+            __syncthreads();
+            for (uint32_t i = me; i < n_tile; i += 4 * THREADS) {
                 uint32_t s[4];
 #pragma unroll
-                for (int u = 0; u < 4; ++u) s[u] = i + u * TILE_CELLS < n_tile ? src[i + u * TILE_CELLS] : 0xffffffffu;
+                for (int u = 0; u < 4; ++u) s[u] = i + u * THREADS < n_tile ? src[i + u * THREADS] : 0xffffffffu;
 #pragma unroll
                 for (int u = 0; u < 4; ++u)
                     if (s[u] != 0xffffffffu) atomicAdd(&sm.count[c.keys[s[u]] >> KEY_CELL_SHIFT], 1u);
             }
-            group_sync<GROUPS>();
+            __syncthreads();
             // the cells' first entries, and cursors for the placement below
             if (me < 32) scan_cell_counts(me, sm.count, sm.cells, sm.start);
-            group_sync<GROUPS>();
+            __syncthreads();
             uint32_t *list = c.tmp + begin;
-            for (uint32_t i = me; i < n_tile; i += 4 * TILE_CELLS) {
+            for (uint32_t i = me; i < n_tile; i += 4 * THREADS) {
                 uint32_t s[4], cell[4];
 #pragma unroll
-                for (int u = 0; u < 4; ++u) s[u] = i + u * TILE_CELLS < n_tile ? src[i + u * TILE_CELLS] : 0xffffffffu;
+                for (int u = 0; u < 4; ++u) s[u] = i + u * THREADS < n_tile ? src[i + u * THREADS] : 0xffffffffu;
 #pragma unroll
                 for (int u = 0; u < 4; ++u) cell[u] = s[u] != 0xffffffffu ? c.keys[s[u]] >> KEY_CELL_SHIFT : 0u;
 #pragma unroll
                 for (int u = 0; u < 4; ++u)
                     if (s[u] != 0xffffffffu) list[atomicAdd(&sm.start[cell[u]], 1u)] = s[u];
             }
-            // the list is written (global, read back by this group)
-            if constexpr (GROUPS > 1) __threadfence_block();
-            group_sync<GROUPS>();
+            __syncthreads();  // the list is written (global, read back by this CTA)
             src = list;
         }
         bool ok = true;
@@ -1462,7 +1433,7 @@ __device__ __forceinline__ void p2g_tiles(const Ctx &c0, Stage<CAP> *stages)
                     hi = sm.cells[q1];
                 }
             }
-            ok = p2g_chunk<CAP, GROUPS, LIQ, REC>(c, sm, src, lo, hi);
+            ok = p2g_chunk<CAP, ROLES, LIQ, REC>(c, sm, src, lo, hi);
             if (n_tile > (uint32_t)CAP && q1 == q + 1 && hi < sm.cells[q + 1]) {
                 i0 += (uint32_t)CAP;  // next chunk of the same crowded cell
             } else {
@@ -1474,7 +1445,7 @@ __device__ __forceinline__ void p2g_tiles(const Ctx &c0, Stage<CAP> *stages)
         const uint32_t mask = sm.mask;
         if (me == 0) c.tile_info[tile] = make_uint2(stamp, mask);
         float *out = c.part + (size_t)tile * (ACC_WORDS * RING_NODES);
-        for (int k = me; k < ACC_WORDS * RING_NODES; k += TILE_CELLS) {
+        for (int k = me; k < ACC_WORDS * RING_NODES; k += THREADS) {
             const int word = k / RING_NODES;
             const uint32_t bit = word < 3 ? 1u : (word < 7 ? 2u : 4u);
             if (mask & bit) out[k] = (&sm.acc[0][0])[k];
@@ -1484,11 +1455,17 @@ __device__ __forceinline__ void p2g_tiles(const Ctx &c0, Stage<CAP> *stages)
 
 }  // namespace
 
-template <bool SCENES, int CAP, bool LIQ, bool REC>
-__global__ void __launch_bounds__(TILE_CELLS, 5) k_p2g_gather(Ctx c0)
+// ROLES threads per cell.  One (36 sums in 96 registers, 20 warps per SM) is
+// faster where every SM has its tiles: 1,000,000 particles 41.4 us against 55.2,
+// the second thread repeating the weights.  Two (20 sums, 48 or 64 registers, up to
+// 40 warps) shorten the chain of a tile where tiles are few or crowded:
+// 1,600 particles 7.7 -> 6.9 us, 24 tanks in one solver 29.5 -> 27.0 us per
+// launch, 512 tanks 812 -> 795 us per substep.
+template <bool SCENES, int CAP, int ROLES, bool LIQ, bool REC>
+__global__ void __launch_bounds__(ROLES *TILE_CELLS, ROLES == 1 || REC ? 5 : 4) k_p2g_gather(Ctx c0)
 {
     extern __shared__ __align__(16) unsigned char dsm[];
-    p2g_tiles<SCENES, CAP, 1, LIQ, REC>(c0, reinterpret_cast<Stage<CAP> *>(dsm));
+    p2g_tiles<SCENES, CAP, ROLES, LIQ, REC>(c0, *reinterpret_cast<Stage<CAP> *>(dsm));
 }
 
 namespace {
@@ -2583,21 +2560,20 @@ static_assert(SUBSTEP_THREADS == ALLOC_THREADS && SUBSTEP_THREADS == 2 * TILE_CE
 // CTAs (at most as many as fit on the GPU at once, so every CTA runs to each
 // barrier): the tile allocation chunks over the CTAs (k_tile_alloc), then the
 // bucketing of every slot with the start of the substep (k_tile_scatter),
-// then P2G over the listed tiles with two tiles at a time per CTA, one per
-// 128-thread group (k_p2g_gather), then the grid update and G2P over the
-// same list (k_g2p_tile), with a grid barrier between phases.  The phases
-// run the four kernels' device functions, so the two forms are
-// bit-identical.  Shared memory is one dynamic buffer: the two P2G stages in
-// that phase, the G2P arrays in the next.
+// then P2G over the listed tiles (k_p2g_gather), then the grid update and G2P
+// over the same list (k_g2p_tile), with a grid barrier between phases.  The
+// phases run the four kernels' device functions, so the two forms are
+// bit-identical.  Shared memory is one dynamic buffer: the P2G stage in that
+// phase, the G2P arrays in the next.
 template <bool SCENES, int CAP, bool LIQ>
-__global__ void __launch_bounds__(SUBSTEP_THREADS, CAP == STAGE_CAP ? 2 : 3) k_substep(Ctx c0)
+__global__ void __launch_bounds__(SUBSTEP_THREADS, LIQ ? 4 : 3) k_substep(Ctx c0)
 {
     extern __shared__ __align__(16) unsigned char dsm[];
     for (uint32_t b = blockIdx.x; b < c0.alloc_chunks; b += gridDim.x) alloc_chunk(c0, b);
     if (!grid_barrier(c0, 0u)) return;
     scatter_quads(c0, blockIdx.x * SUBSTEP_THREADS + (threadIdx.x & ~31u), gridDim.x * SUBSTEP_THREADS);
     if (!grid_barrier(c0, 1u)) return;
-    p2g_tiles<SCENES, CAP, 2, LIQ, false>(c0, reinterpret_cast<Stage<CAP> *>(dsm));
+    p2g_tiles<SCENES, CAP, 2, LIQ, false>(c0, *reinterpret_cast<Stage<CAP> *>(dsm));
     if (!grid_barrier(c0, 2u)) return;
     g2p_tiles<SCENES, false, LIQ, false>(c0, *reinterpret_cast<G2PShared *>(dsm));
 }
@@ -2607,7 +2583,7 @@ size_t p2g_shared_bytes(int cap)
     return cap == STAGE_CAP_NARROW ? sizeof(Stage<STAGE_CAP_NARROW>) : sizeof(Stage<STAGE_CAP>);
 }
 
-size_t substep_shared_bytes(int cap) { return std::max(2 * p2g_shared_bytes(cap), sizeof(G2PShared)); }
+size_t substep_shared_bytes(int cap) { return std::max(p2g_shared_bytes(cap), sizeof(G2PShared)); }
 
 // The start of a substep of the fixed-point path (k_tile_alloc starts those
 // of the default path): begin_substep for every scene.
@@ -3587,22 +3563,38 @@ __global__ void k_probe_deformation(const float4 *F, const float4 *C, float dt, 
     substeps[i] = t.substeps;
 }
 
-template __global__ void k_p2g_gather<false, STAGE_CAP, false, false>(Ctx);
-template __global__ void k_p2g_gather<true, STAGE_CAP, false, false>(Ctx);
-template __global__ void k_p2g_gather<false, STAGE_CAP_NARROW, false, false>(Ctx);
-template __global__ void k_p2g_gather<true, STAGE_CAP_NARROW, false, false>(Ctx);
-template __global__ void k_p2g_gather<false, STAGE_CAP, true, false>(Ctx);
-template __global__ void k_p2g_gather<true, STAGE_CAP, true, false>(Ctx);
-template __global__ void k_p2g_gather<false, STAGE_CAP_NARROW, true, false>(Ctx);
-template __global__ void k_p2g_gather<true, STAGE_CAP_NARROW, true, false>(Ctx);
-template __global__ void k_p2g_gather<false, STAGE_CAP, false, true>(Ctx);
-template __global__ void k_p2g_gather<true, STAGE_CAP, false, true>(Ctx);
-template __global__ void k_p2g_gather<false, STAGE_CAP_NARROW, false, true>(Ctx);
-template __global__ void k_p2g_gather<true, STAGE_CAP_NARROW, false, true>(Ctx);
-template __global__ void k_p2g_gather<false, STAGE_CAP, true, true>(Ctx);
-template __global__ void k_p2g_gather<true, STAGE_CAP, true, true>(Ctx);
-template __global__ void k_p2g_gather<false, STAGE_CAP_NARROW, true, true>(Ctx);
-template __global__ void k_p2g_gather<true, STAGE_CAP_NARROW, true, true>(Ctx);
+template __global__ void k_p2g_gather<false, STAGE_CAP, 1, false, false>(Ctx);
+template __global__ void k_p2g_gather<false, STAGE_CAP, 1, false, true>(Ctx);
+template __global__ void k_p2g_gather<false, STAGE_CAP, 1, true, false>(Ctx);
+template __global__ void k_p2g_gather<false, STAGE_CAP, 1, true, true>(Ctx);
+template __global__ void k_p2g_gather<false, STAGE_CAP, 2, false, false>(Ctx);
+template __global__ void k_p2g_gather<false, STAGE_CAP, 2, false, true>(Ctx);
+template __global__ void k_p2g_gather<false, STAGE_CAP, 2, true, false>(Ctx);
+template __global__ void k_p2g_gather<false, STAGE_CAP, 2, true, true>(Ctx);
+template __global__ void k_p2g_gather<false, STAGE_CAP_NARROW, 1, false, false>(Ctx);
+template __global__ void k_p2g_gather<false, STAGE_CAP_NARROW, 1, false, true>(Ctx);
+template __global__ void k_p2g_gather<false, STAGE_CAP_NARROW, 1, true, false>(Ctx);
+template __global__ void k_p2g_gather<false, STAGE_CAP_NARROW, 1, true, true>(Ctx);
+template __global__ void k_p2g_gather<false, STAGE_CAP_NARROW, 2, false, false>(Ctx);
+template __global__ void k_p2g_gather<false, STAGE_CAP_NARROW, 2, false, true>(Ctx);
+template __global__ void k_p2g_gather<false, STAGE_CAP_NARROW, 2, true, false>(Ctx);
+template __global__ void k_p2g_gather<false, STAGE_CAP_NARROW, 2, true, true>(Ctx);
+template __global__ void k_p2g_gather<true, STAGE_CAP, 1, false, false>(Ctx);
+template __global__ void k_p2g_gather<true, STAGE_CAP, 1, false, true>(Ctx);
+template __global__ void k_p2g_gather<true, STAGE_CAP, 1, true, false>(Ctx);
+template __global__ void k_p2g_gather<true, STAGE_CAP, 1, true, true>(Ctx);
+template __global__ void k_p2g_gather<true, STAGE_CAP, 2, false, false>(Ctx);
+template __global__ void k_p2g_gather<true, STAGE_CAP, 2, false, true>(Ctx);
+template __global__ void k_p2g_gather<true, STAGE_CAP, 2, true, false>(Ctx);
+template __global__ void k_p2g_gather<true, STAGE_CAP, 2, true, true>(Ctx);
+template __global__ void k_p2g_gather<true, STAGE_CAP_NARROW, 1, false, false>(Ctx);
+template __global__ void k_p2g_gather<true, STAGE_CAP_NARROW, 1, false, true>(Ctx);
+template __global__ void k_p2g_gather<true, STAGE_CAP_NARROW, 1, true, false>(Ctx);
+template __global__ void k_p2g_gather<true, STAGE_CAP_NARROW, 1, true, true>(Ctx);
+template __global__ void k_p2g_gather<true, STAGE_CAP_NARROW, 2, false, false>(Ctx);
+template __global__ void k_p2g_gather<true, STAGE_CAP_NARROW, 2, false, true>(Ctx);
+template __global__ void k_p2g_gather<true, STAGE_CAP_NARROW, 2, true, false>(Ctx);
+template __global__ void k_p2g_gather<true, STAGE_CAP_NARROW, 2, true, true>(Ctx);
 template __global__ void k_substep<false, STAGE_CAP, false>(Ctx);
 template __global__ void k_substep<true, STAGE_CAP, false>(Ctx);
 template __global__ void k_substep<false, STAGE_CAP_NARROW, false>(Ctx);

@@ -185,9 +185,9 @@ __global__ void k_tile_count(Ctx c);
 __global__ void k_tile_alloc(Ctx c);
 __global__ void k_tile_scatter(Ctx c);
 // SCENES: the solver holds several scenes; CAP: particles staged at once;
-// LIQ: every material is water or oil; REC: the records variant (P2G reads
+// ROLES: threads per cell of a tile; LIQ: every material is water or oil; REC: the records variant (P2G reads
 // the records G2P wrote instead of preparing each particle from its state)
-template <bool SCENES, int CAP, bool LIQ, bool REC>
+template <bool SCENES, int CAP, int ROLES, bool LIQ, bool REC>
 __global__ void k_p2g_gather(Ctx c);
 // The whole substep of the default path in one cooperative launch: tile
 // allocation, bucketing, P2G and G2P, separated by grid barriers whose waits

@@ -142,6 +142,7 @@ struct mpm_solver {
     float2 *body_vel = nullptr;
     uint32_t *bonds = nullptr, *topology = nullptr, *endpoints = nullptr;
     uint32_t n_endpoints = 0, fracture_particles = 0, fracture_incidence = 0;
+    unsigned sms = 1;
     unsigned p2g_ctas = 1, g2p_ctas = 1;  // persistent grids of the default path's P2G and G2P kernels
     // the default path's substep variant: one cooperative launch (k_substep)
     // or four launches, the P2G stage capacity, k_substep's persistent grid
@@ -397,28 +398,29 @@ const void *substep_kernel(bool scenes, int cap, bool liq)
     return scenes ? (const void *)k_substep<true, STAGE_CAP, false> : (const void *)k_substep<false, STAGE_CAP, false>;
 }
 
-template <bool REC>
-const void *p2g_kernel_rec(bool scenes, int cap, bool liq)
+template <bool SCENES, int ROLES>
+const void *p2g_kernel_of(int cap, bool liq, bool rec)
 {
-    if (liq) {
-        if (cap == STAGE_CAP_NARROW)
-            return scenes ? (const void *)k_p2g_gather<true, STAGE_CAP_NARROW, true, REC>
-                          : (const void *)k_p2g_gather<false, STAGE_CAP_NARROW, true, REC>;
-        return scenes ? (const void *)k_p2g_gather<true, STAGE_CAP, true, REC>
-                      : (const void *)k_p2g_gather<false, STAGE_CAP, true, REC>;
+    if (cap == STAGE_CAP_NARROW) {
+        if (liq)
+            return rec ? (const void *)k_p2g_gather<SCENES, STAGE_CAP_NARROW, ROLES, true, true>
+                       : (const void *)k_p2g_gather<SCENES, STAGE_CAP_NARROW, ROLES, true, false>;
+        return rec ? (const void *)k_p2g_gather<SCENES, STAGE_CAP_NARROW, ROLES, false, true>
+                   : (const void *)k_p2g_gather<SCENES, STAGE_CAP_NARROW, ROLES, false, false>;
     }
-    if (cap == STAGE_CAP_NARROW)
-        return scenes ? (const void *)k_p2g_gather<true, STAGE_CAP_NARROW, false, REC>
-                      : (const void *)k_p2g_gather<false, STAGE_CAP_NARROW, false, REC>;
-    return scenes ? (const void *)k_p2g_gather<true, STAGE_CAP, false, REC>
-                  : (const void *)k_p2g_gather<false, STAGE_CAP, false, REC>;
+    if (liq)
+        return rec ? (const void *)k_p2g_gather<SCENES, STAGE_CAP, ROLES, true, true>
+                   : (const void *)k_p2g_gather<SCENES, STAGE_CAP, ROLES, true, false>;
+    return rec ? (const void *)k_p2g_gather<SCENES, STAGE_CAP, ROLES, false, true>
+               : (const void *)k_p2g_gather<SCENES, STAGE_CAP, ROLES, false, false>;
 }
 
-// The k_p2g_gather instantiation for the scene count, stage capacity,
-// material set and records variant.
-const void *p2g_kernel(bool scenes, int cap, bool liq, bool rec)
+// The k_p2g_gather instantiation for the scene count, stage capacity, threads
+// per cell, material set and records variant.
+const void *p2g_kernel(bool scenes, int cap, int roles, bool liq, bool rec)
 {
-    return rec ? p2g_kernel_rec<true>(scenes, cap, liq) : p2g_kernel_rec<false>(scenes, cap, liq);
+    if (scenes) return roles == 1 ? p2g_kernel_of<true, 1>(cap, liq, rec) : p2g_kernel_of<true, 2>(cap, liq, rec);
+    return roles == 1 ? p2g_kernel_of<false, 1>(cap, liq, rec) : p2g_kernel_of<false, 2>(cap, liq, rec);
 }
 
 // Whether the substeps of this solver run as one k_substep launch each:
@@ -434,6 +436,15 @@ bool runs_liquid(const mpm_solver *s)
     for (const Material &m : s->mats)
         if (m.model != MODEL_WATER && m.model != MODEL_OIL) return false;
     return true;
+}
+
+// Threads per cell of P2G (k_p2g_gather gives both sides' times): two for
+// several scenes, whose crowded tiles set the pace, and for one scene of up to
+// a full tile per SM (48,000 particles of six materials: 8.2 -> 7.8 us; at
+// 150,000 the two are equal, above it one is faster).
+int p2g_roles(const mpm_solver *s)
+{
+    return s->n_scenes > 1 || s->n <= 640u * s->sms ? 2 : 1;
 }
 
 // Enqueues k_substep as a cooperative launch (every CTA resident at once).
@@ -457,19 +468,16 @@ cudaError_t launch_substep(mpm_solver *s, const Ctx &c)
 // device; the attributes are per function).
 cudaError_t configure_variant_kernels()
 {
-    const int caps[2] = {STAGE_CAP, STAGE_CAP_NARROW};
-    for (int cap : caps) {
-        for (int scenes = 0; scenes < 2; ++scenes) {
-            const void *fns[6] = {p2g_kernel(scenes != 0, cap, false, false), p2g_kernel(scenes != 0, cap, true, false),
-                                  p2g_kernel(scenes != 0, cap, false, true),  p2g_kernel(scenes != 0, cap, true, true),
-                                  substep_kernel(scenes != 0, cap, false), substep_kernel(scenes != 0, cap, true)};
-            const size_t bytes[6] = {p2g_shared_bytes(cap), p2g_shared_bytes(cap), p2g_shared_bytes(cap),
-                                     p2g_shared_bytes(cap), substep_shared_bytes(cap), substep_shared_bytes(cap)};
-            for (int k = 0; k < 6; ++k) {
-                cudaError_t e = cudaFuncSetAttribute(fns[k], cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes[k]);
-                if (e == cudaSuccess) e = cudaFuncSetAttribute(fns[k], cudaFuncAttributePreferredSharedMemoryCarveout, 100);
-                if (e != cudaSuccess) return e;
-            }
+    auto configure = [](const void *fn, size_t bytes) {
+        const cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+        return e == cudaSuccess ? cudaFuncSetAttribute(fn, cudaFuncAttributePreferredSharedMemoryCarveout, 100) : e;
+    };
+    for (int cap : {STAGE_CAP, STAGE_CAP_NARROW}) {
+        for (int v = 0; v < 16; ++v) {
+            const bool scenes = (v & 1) != 0, liq = (v & 2) != 0, rec = (v & 4) != 0;
+            cudaError_t e = configure(p2g_kernel(scenes, cap, (v & 8) ? 2 : 1, liq, rec), p2g_shared_bytes(cap));
+            if (e == cudaSuccess && v < 4) e = configure(substep_kernel(scenes, cap, liq), substep_shared_bytes(cap));
+            if (e != cudaSuccess) return e;
         }
     }
     return cudaSuccess;
@@ -478,8 +486,8 @@ cudaError_t configure_variant_kernels()
 // CTAs per SM of the P2G kernel and of k_substep for stage capacity `cap`.
 cudaError_t variant_occupancy(int cap, int *per_sm_p2g, int *per_sm_substep)
 {
-    cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(per_sm_p2g, p2g_kernel(false, cap, false, false), TILE_CELLS,
-                                                                  p2g_shared_bytes(cap));
+    cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(
+        per_sm_p2g, p2g_kernel(false, cap, 1, false, false), TILE_CELLS, p2g_shared_bytes(cap));
     if (e == cudaSuccess)
         e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(per_sm_substep, substep_kernel(false, cap, false), SUBSTEP_THREADS,
                                                           substep_shared_bytes(cap));
@@ -520,8 +528,8 @@ void enqueue_substep(mpm_solver *s, int parity)
         mark(K_TILE_SCATTER);
         {
             void *args[] = {const_cast<Ctx *>(&c)};
-            cudaLaunchKernel(p2g_kernel(s->n_scenes > 1, s->stage_cap, runs_liquid(s), uses_records(s)), dim3(s->p2g_ctas),
-                             dim3(TILE_CELLS), args,
+            cudaLaunchKernel(p2g_kernel(s->n_scenes > 1, s->stage_cap, p2g_roles(s), runs_liquid(s), uses_records(s)),
+                             dim3(s->p2g_ctas), dim3(p2g_roles(s) * TILE_CELLS), args,
                              p2g_shared_bytes(s->stage_cap), s->stream);
         }
         mark(K_P2G_GATHER);
@@ -1088,6 +1096,7 @@ int create_impl(const mpm_config *configs, uint32_t n_scenes, const uint32_t *co
             cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm_g2p, k_g2p_tile<false, false, false, false>, G2P_THREADS, 0) !=
                 cudaSuccess)
             return fail(set_error(MPM_ERR_CUDA, "occupancy query failed"));
+        s->sms = (unsigned)sms;
         s->p2g_ctas = (unsigned)std::max<size_t>(1, std::min<size_t>(n_tiles, (size_t)sms * std::max(1, per_sm_p2g)));
         s->g2p_ctas = (unsigned)std::max<size_t>(1, std::min<size_t>(n_tiles, (size_t)sms * std::max(1, per_sm_g2p)));
         s->substep_max_ctas = (unsigned)std::max(1, sms * per_sm_substep);
