@@ -2,8 +2,9 @@
 //
 // Substep, default P2G (the role of the reference's gather path,
 // src/lib/mpm/kernels/solver.ts:1465-1570):
-//   k_tile_alloc (starts the substep) -> k_tile_scatter -> k_p2g_gather
-//   -> k_g2p_tile (grid update + G2P + next substep's tile counts)
+//   k_tile_bucket (one scene of few tiles; starts the substep) or k_tile_alloc
+//   -> k_tile_scatter (starts it) -> k_p2g_gather -> k_g2p_tile (grid update +
+//   G2P + next substep's tile counts)
 //   (k_begin_batch and k_tile_count run once at the start of a batch);
 //   or the same four phases in one cooperative launch, k_substep, with grid
 //   barriers between them
@@ -249,9 +250,9 @@ __device__ __forceinline__ uint32_t listed_count(const Ctx &c)
 
 __device__ __forceinline__ uint32_t heavy_count(const Ctx &c) { return __ldcg(c.work + WORK_HEAVY + c.parity); }
 
-__device__ __forceinline__ const uint32_t *listed_tile(const Ctx &c, uint32_t item, uint32_t heavy)
+__device__ __forceinline__ const uint4 *listed_tile(const Ctx &c, const uint4 *list, uint32_t item, uint32_t heavy)
 {
-    return item < heavy ? c.active_tiles + (c.n_tiles - 1u - item) : c.active_tiles + (item - heavy);
+    return item < heavy ? list + (c.n_tiles - 1u - item) : list + (item - heavy);
 }
 
 // Whether the scene takes part in the current substep: no status raised and
@@ -346,6 +347,15 @@ __device__ __forceinline__ void cp_async(void *dst, const void *src)
         asm volatile("cp.async.ca.shared.global [%0], [%1], %2;\n" ::"r"(d), "l"(src), "n"(N) : "memory");
 }
 
+// The start of a kernel of the substep chain: its CTAs may have been started
+// while the last CTAs of the kernel before it ended (a programmatic launch;
+// without one there is nothing to wait for); that kernel's results are complete
+// and visible from here on.  2-5 % of a substep at every size measured (1,600
+// particles 22.3 -> 21.8 us, 150,000 32.4 -> 31.0, 1,000,000 103.2 -> 103.0).
+// Letting the next kernel's CTAs start with this one's costs more than it gives:
+// they hold slots (1,000,000: 115.7 us).
+__device__ __forceinline__ void follow() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
 __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;\n" ::: "memory"); }
 
 __device__ __forceinline__ uint32_t warp_sum(uint32_t v)
@@ -411,6 +421,7 @@ __device__ __forceinline__ uint32_t warp_count(uint32_t *cell_count, uint32_t ke
 // after it) and the tile lists.
 __global__ void k_begin_batch(Ctx c, uint32_t reset_progress)
 {
+    follow();
     for (uint32_t s = blockIdx.x * blockDim.x + threadIdx.x; s < c.n_scenes; s += gridDim.x * blockDim.x) {
         uint32_t *counters = c.dyn + (size_t)s * SCENE_WORDS + 32;
         if (reset_progress) counters[COUNTER_PROGRESS] = 0u;
@@ -425,6 +436,7 @@ __global__ void k_begin_batch(Ctx c, uint32_t reset_progress)
         c.work[WORK_ACTIVE + 1] = 0u;
         c.work[WORK_HEAVY] = 0u;
         c.work[WORK_HEAVY + 1] = 0u;
+        c.work[WORK_TICKET] = 0u;
         c.work[WORK_BARRIER] = 0u;  // an abandoned launch may have left arrivals
         c.work[WORK_ABORT] = 0u;
     }
@@ -764,6 +776,7 @@ __device__ __forceinline__ uint32_t bucket_key(uint32_t tile, int bx, int by)
 // (later substeps get them from G2P).
 __global__ void k_tile_count(Ctx c0)
 {
+    follow();
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     const Ctx c = scene_ctx(c0, c0.n_scenes == 1u || i >= c0.n ? 0u : scene_of_slot(c0, i));
     const StepParams &P = *c.P;
@@ -927,16 +940,21 @@ __device__ __forceinline__ void alloc_chunk(const Ctx &c0, uint32_t b)
             // light tiles from the front of the list, heavy ones from its end
 #pragma unroll
             for (int k = 0; k < ALLOC_ITEMS; ++k) {
+                const uint4 item = make_uint4(P.tile_base + first + k, r[k].x, v[k], 0u);
                 if (v[k] > HEAVY_TILE)
-                    c.active_tiles[c0.n_tiles - 1u - heavy_slot++] = P.tile_base + first + k;
+                    c.active_tiles[c0.n_tiles - 1u - heavy_slot++] = item;
                 else if (v[k] != 0u)
-                    c.active_tiles[slot++] = P.tile_base + first + k;
+                    c.active_tiles[slot++] = item;
             }
         }
     }
 }
 
-__global__ void __launch_bounds__(ALLOC_THREADS) k_tile_alloc(Ctx c0) { alloc_chunk(c0, blockIdx.x); }
+__global__ void __launch_bounds__(ALLOC_THREADS) k_tile_alloc(Ctx c0)
+{
+    follow();
+    alloc_chunk(c0, blockIdx.x);
+}
 
 // Starts the substep of every scene (the first threads of CTA 0) and buckets
 // the slots 4q .. 4q + 3 of every quad q = q0 + lane for q0 from `first`
@@ -999,7 +1017,99 @@ __device__ __forceinline__ void scatter_quads(const Ctx &c, uint32_t first, uint
 // scene takes part.
 __global__ void k_tile_scatter(Ctx c)
 {
+    follow();
     scatter_quads(c, blockIdx.x * blockDim.x + (threadIdx.x & ~31u), gridDim.x * blockDim.x);
+}
+
+// k_tile_alloc and k_tile_scatter as one kernel, for one scene of at most
+// BUCKET_TILES tiles: every CTA scans the counts of all tiles itself (the
+// same answer in each, in tile order), so that it can place its slots, four
+// per thread, without waiting for another; CTA 0 also writes the tile list.
+// The counts are zeroed by P2G, tile by tile, once every CTA has read them.
+// With `divided` it also lists what G2P takes: a tile in up to G2P_MAX_PARTS
+// items of whole rounds of G2P's threads.  A CTA that takes one evaluates the
+// tile's ring like the CTAs of the others and moves its share of the
+// particles: fewer rounds where the tiles are fewer than the SMs (1,600
+// particles: G2P 12.1 -> 10.3 us; items of 128 or 64 particles change nothing
+// more, a round then takes its chain of dependent instructions).
+// The last CTA to have read whether the scene runs starts the substep
+// (begin_substep).  What it costs is latency: the counts, keys and ranks come
+// in together, then the scan, then the stores; a substep of 1,600 particles
+// fell from 21.8 to 21.2 us against the two kernels, one of 150,000 from 31.0 to
+// 30.5 us.
+__global__ void __launch_bounds__(BUCKET_THREADS) k_tile_bucket(Ctx c)
+{
+    follow();
+    __shared__ uint32_t s_first[BUCKET_TILES];  // first bucket entry per tile
+    __shared__ bool s_runs;
+    const uint32_t n_tiles = c.P->scene_tiles;
+    const uint32_t t0 = threadIdx.x * 4u;
+    const uint32_t i = (blockIdx.x * BUCKET_THREADS + threadIdx.x) * 4u;
+    uint32_t v[4], key[4], rank[4];
+    if (t0 + 4u <= n_tiles) {
+        const uint4 a = __ldcg(reinterpret_cast<const uint4 *>(c.tile_count + t0));
+        v[0] = a.x, v[1] = a.y, v[2] = a.z, v[3] = a.w;
+    } else {
+#pragma unroll
+        for (int k = 0; k < 4; ++k) v[k] = t0 + k < n_tiles ? __ldcg(c.tile_count + t0 + k) : 0u;
+    }
+    if (i + 4u <= c.n) {
+        const uint4 a = __ldcg(reinterpret_cast<const uint4 *>(c.keys + i));
+        const uint4 b = __ldcg(reinterpret_cast<const uint4 *>(c.ranks + i));
+        key[0] = a.x, key[1] = a.y, key[2] = a.z, key[3] = a.w;
+        rank[0] = b.x, rank[1] = b.y, rank[2] = b.z, rank[3] = b.w;
+    } else {
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            key[k] = i + k < c.n ? __ldcg(c.keys + i + k) : 0u;
+            rank[k] = i + k < c.n ? __ldcg(c.ranks + i + k) : 0u;
+        }
+    }
+    if (threadIdx.x == 0) s_runs = substep_runs(c);
+    // particles in the high word; listed tiles and G2P items (at most 4096 and
+    // 16384) in the low and high halves of the low word
+    unsigned long long mine = 0ull, total;
+    uint32_t parts[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        parts[k] = c.divided ? min((v[k] + G2P_THREADS - 1u) / G2P_THREADS, G2P_MAX_PARTS) : (v[k] != 0u ? 1u : 0u);
+        mine += ((unsigned long long)v[k] << 32) | (parts[k] << 16) | (v[k] != 0u ? 1u : 0u);
+    }
+    const unsigned long long offset = block_exclusive_scan<BUCKET_THREADS, unsigned long long>(mine, total);
+    const bool runs = s_runs;
+    uint32_t at = (uint32_t)(offset >> 32);
+    uint32_t slot = (uint32_t)offset & 0xffffu, item = ((uint32_t)offset >> 16) & 0xffffu;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        s_first[t0 + k] = at;
+        if (blockIdx.x == 0 && runs && v[k] != 0u) {
+            c.active_tiles[slot++] = make_uint4(t0 + k, at, v[k], 0u);
+            if (c.divided) {
+                // parts of whole rounds of G2P's threads
+                const uint32_t rounds = (v[k] + G2P_THREADS - 1u) / G2P_THREADS;
+                const uint32_t size = (rounds + parts[k] - 1u) / parts[k] * G2P_THREADS;
+                for (uint32_t p = 0; p < parts[k]; ++p) {
+                    const uint32_t from = min(p * size, v[k]);
+                    c.g2p_items[item++] = make_uint4(t0 + k, at + from, min(size, v[k] - from), 0u);
+                }
+            }
+        }
+        at += v[k];
+    }
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        c.work[WORK_ACTIVE + c.parity] = runs ? (uint32_t)total & 0xffffu : 0u;
+        c.work[WORK_HEAVY + c.parity] = 0u;
+        c.work[WORK_ITEMS + c.parity] = runs ? ((uint32_t)total >> 16) & 0xffffu : 0u;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < 4; ++k)
+        if (runs && i + k < c.n) c.perm[s_first[key[k] & KEY_TILE_MASK] + rank[k]] = i + k;
+    // every CTA comes here with its answer to whether the scene runs
+    if (threadIdx.x == 0 && (gridDim.x == 1u || atomicAdd(c.work + WORK_TICKET, 1u) == gridDim.x - 1u)) {
+        c.work[WORK_TICKET] = 0u;
+        begin_substep(c);
+    }
 }
 
 namespace {
@@ -1354,6 +1464,9 @@ __device__ __forceinline__ void p2g_tiles(const Ctx &c0, Stage<CAP> &sm)
 {
     constexpr uint32_t THREADS = ROLES * TILE_CELLS;
     const uint32_t me = threadIdx.x;
+    // one scene: the first light tile this CTA takes, fetched with the counts
+    uint4 light = make_uint4(0u, 0u, 0u, 0u);
+    if constexpr (!SCENES) light = __ldcg(c0.active_tiles + min(blockIdx.x, c0.n_tiles - 1u));
     const uint32_t n_active = listed_count(c0), n_heavy = heavy_count(c0);
     // several scenes: each CTA claims its next tile (the heavy ones are
     // listed first), which evens out tiles of very different sizes; one scene
@@ -1369,16 +1482,16 @@ __device__ __forceinline__ void p2g_tiles(const Ctx &c0, Stage<CAP> &sm)
         }
     };
     for (uint32_t item = SCENES ? next(0u) : blockIdx.x; item < n_active; item = next(item)) {
-        const uint32_t tile = __ldcg(listed_tile(c0, item, n_heavy));
+        const uint4 listed = !SCENES && item == blockIdx.x && n_heavy == 0u ? light : __ldcg(listed_tile(c0, c0.active_tiles, item, n_heavy));
+        const uint32_t tile = listed.x, begin = listed.y, n_tile = listed.z;
         const Ctx c = tile_ctx<SCENES>(c0, tile);
         const uint32_t stamp = __ldcg(c.counters + COUNTER_STAMP);
-        const uint2 range = __ldcg(c.tile_range + tile);
-        const uint32_t begin = range.x, n_tile = range.y;
         __syncthreads();  // the previous tile's readers of sm are done
         for (int k = me; k < ACC_WORDS * RING_NODES; k += THREADS) (&sm.acc[0][0])[k] = 0.f;
         if (me == 0) {
             sm.failed = *(volatile uint32_t *)c.status != 0u ? 1 : 0;  // one read for the whole CTA
             sm.mask = 0u;
+            c.tile_count[tile] = 0u;  // G2P counts the next substep's particles from here
         }
         __syncthreads();
         if (sm.failed) continue;  // the scene's substep is rolled back
@@ -1464,6 +1577,7 @@ __device__ __forceinline__ void p2g_tiles(const Ctx &c0, Stage<CAP> &sm)
 template <bool SCENES, int CAP, int ROLES, bool LIQ, bool REC>
 __global__ void __launch_bounds__(ROLES *TILE_CELLS, ROLES == 1 || REC ? 5 : 4) k_p2g_gather(Ctx c0)
 {
+    follow();
     extern __shared__ __align__(16) unsigned char dsm[];
     p2g_tiles<SCENES, CAP, ROLES, LIQ, REC>(c0, *reinterpret_cast<Stage<CAP> *>(dsm));
 }
@@ -1608,6 +1722,7 @@ __device__ __forceinline__ bool add_fixed(const Ctx &c, uint32_t index, float va
 // bit-exactly against a CPU emulation of the same integers.
 __global__ void k_prepare_scatter(Ctx c)
 {
+    follow();
     const StepParams &P = *c.P;
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= P.n_particles) return;
@@ -1658,6 +1773,7 @@ __global__ void k_prepare_scatter(Ctx c)
 // the accumulators are always clean for the next substep.
 __global__ void __launch_bounds__(TILE_NODES) k_fixed_decode(Ctx c)
 {
+    follow();
     const StepParams &P = *c.P;
     const int tx = blockIdx.x, ty = blockIdx.y;
     if (c.tile_stamp[ty * P.tiles_x + tx] != c.counters[COUNTER_STAMP]) return;
@@ -1698,6 +1814,7 @@ __device__ __forceinline__ float2 phase_volume(const Ctx &c, int hx, int hy, uin
 // sums of touched tiles.
 __global__ void __launch_bounds__(TILE_NODES) k_grid_update(Ctx c)
 {
+    follow();
     const StepParams &P = *c.P;
     const int tx = blockIdx.x, ty = blockIdx.y;
     const uint32_t stamp = c.counters[COUNTER_STAMP];
@@ -2141,6 +2258,7 @@ __device__ __forceinline__ bool g2p_particle(const Ctx &c, const ParticleIn &in,
 // particle's new base cell for the next substep's sort.
 __global__ void k_g2p(Ctx c)
 {
+    follow();
     const StepParams &P = *c.P;
     const uint32_t d = blockIdx.x * blockDim.x + threadIdx.x;
     const bool in_range = d < P.n_particles;
@@ -2218,11 +2336,11 @@ __device__ __forceinline__ void stage_chunk(const Ctx &c, const uint32_t *entrie
 // theirs, so their G2P flags can join the status of that substep.
 // Shared memory of the G2P phase.
 struct G2PShared {
-    // per buffer parity: the tile, its bucket range and its 3x3 neighbours'
-    // (stamp, mask); with one scene the next tile's are copied in while this
-    // one's particles move, and the index of the one after it
-    uint32_t tile[2];
-    uint2 range[2];
+    // per buffer parity: the tile with its bucket range (its entry in the tile
+    // list) and its 3x3 neighbours' (stamp, mask); with one scene the next
+    // tile's are copied in while this one's particles move, and the list entry
+    // of the one after it
+    uint4 item[2];
     uint2 infos[2][9];
     // with one scene: the next tile's first G2P_STAGE bucket entries and the
     // scene's status words, copied in while this tile's particles move
@@ -2245,8 +2363,7 @@ struct G2PShared {
 template <bool SCENES, bool BODIES, bool LIQ, bool REC>
 __device__ __forceinline__ void g2p_tiles(const Ctx &c0, G2PShared &sh)
 {
-    uint32_t *const s_tile = sh.tile;
-    uint2 *const s_range = sh.range;
+    uint4 *const s_item = sh.item;
     uint2(*const s_infos)[9] = sh.infos;
     uint32_t(*const s_perm)[G2P_STAGE] = sh.perm;
     uint32_t(*const s_status)[4] = sh.status;
@@ -2259,11 +2376,20 @@ __device__ __forceinline__ void g2p_tiles(const Ctx &c0, G2PShared &sh)
     float2 *const p_pos = sh.pos;
     float *const p_vol = sh.vol_in, *const p_pvol = sh.pvol_in, *const p_damage = sh.damage;
     uint32_t *const p_mat = sh.mat, *const p_orig = sh.orig;
-    const uint32_t n_active = listed_count(c0), n_heavy = heavy_count(c0);
-    if constexpr (!SCENES) {
+    uint32_t n_items, n_heavy;
+    auto item_at = [&](uint32_t v) { return listed_tile(c0, c0.g2p_items, v, n_heavy); };
+    if constexpr (SCENES) {
+        n_items = listed_count(c0), n_heavy = heavy_count(c0);
+    } else {
+        // the first item of this CTA if no tile is heavy, fetched with the
+        // counts; every thread stores the entry that it reads below
+        uint4 first = __ldcg(c0.g2p_items + min(blockIdx.x, c0.n_tiles * (c0.divided ? G2P_MAX_PARTS : 1u) - 1u));
+        n_items = c0.divided ? __ldcg(c0.work + WORK_ITEMS + c0.parity) : listed_count(c0);
+        n_heavy = c0.divided ? 0u : heavy_count(c0);
+        if (n_heavy != 0u && blockIdx.x < n_items) first = __ldcg(item_at(blockIdx.x));
+        s_item[0] = first;
         // visible after the first iteration's barrier
-        if (threadIdx.x == 0 && blockIdx.x + gridDim.x < n_active)
-            s_tile[1] = *listed_tile(c0, blockIdx.x + gridDim.x, n_heavy);
+        if (threadIdx.x == 0 && blockIdx.x + gridDim.x < n_items) s_item[1] = *item_at(blockIdx.x + gridDim.x);
     }
     // several scenes: each CTA claims its next tile (the heavy ones are listed
     // first); one scene: a fixed stride, with the next tile's data copied in
@@ -2278,13 +2404,14 @@ __device__ __forceinline__ void g2p_tiles(const Ctx &c0, G2PShared &sh)
         }
     };
     uint32_t it = 0;
-    for (uint32_t item = SCENES ? next(0u) : blockIdx.x; item < n_active; item = next(item), ++it) {
+    for (uint32_t item = SCENES ? next(0u) : blockIdx.x; item < n_items; item = next(item), ++it) {
         const uint32_t buf = it & 1u;
         const bool fetched = !SCENES && it > 0u;  // copied in during the previous tile
         uint2 *const info = s_infos[buf];
         // (the copies read here landed, and were made visible by a barrier,
         // during the previous tile)
-        const uint32_t tile = fetched ? s_tile[buf] : *listed_tile(c0, item, n_heavy);
+        const uint4 listed = SCENES ? __ldcg(item_at(item)) : s_item[buf];
+        const uint32_t tile = listed.x;
         const uint32_t nb = buf ^ 1u;
         const Ctx c = tile_ctx<SCENES>(c0, tile);
         const StepParams &P = *c.P;
@@ -2293,11 +2420,11 @@ __device__ __forceinline__ void g2p_tiles(const Ctx &c0, G2PShared &sh)
         // during this tile (it has no particle phase when its scene failed)
         auto prefetch_next = [&]() {
             if constexpr (!SCENES) {
-                if (item + gridDim.x < n_active) {
-                    const uint2 nr = s_range[nb];
-                    const uint32_t count = min(nr.y, (uint32_t)G2P_STAGE);
+                if (item + gridDim.x < n_items) {
+                    const uint4 next_item = s_item[nb];
+                    const uint32_t count = min(next_item.z, (uint32_t)G2P_STAGE);
                     for (uint32_t i = threadIdx.x; i < count; i += G2P_THREADS)
-                        cp_async<4>(&s_perm[nb][i], &c.perm[nr.x + i]);
+                        cp_async<4>(&s_perm[nb][i], &c.perm[next_item.y + i]);
                     if (threadIdx.x == G2P_THREADS - 1) cp_async<16>(&s_status[nb][0], c.status);
                 }
             }
@@ -2307,8 +2434,7 @@ __device__ __forceinline__ void g2p_tiles(const Ctx &c0, G2PShared &sh)
         const uint32_t local = tile - P.tile_base;
         const int tx = (int)(local % P.tiles_x), ty = (int)(local / P.tiles_x);
         const int x0 = tx * TILE_X, y0 = ty * TILE_Y;
-        const uint2 range = fetched ? s_range[buf] : c.tile_range[tile];
-        const uint32_t begin = range.x, end = range.x + range.y;
+        const uint32_t begin = listed.y, end = listed.y + listed.z;
         if (fetched) cp_async_wait_all();  // this tile's entries and status words (visible after the barrier)
         __syncthreads();  // readers of the previous tile's shared data are done
         if (!fetched && threadIdx.x < 9) {
@@ -2326,25 +2452,20 @@ __device__ __forceinline__ void g2p_tiles(const Ctx &c0, G2PShared &sh)
                     p_vol, p_pvol, p_damage, p_mat, p_orig);
         __syncthreads();
         if constexpr (!SCENES) {
-            // the next tile's range and neighbour records (its index came in
-            // during the previous tile) and the index of the tile after it;
+            // the next tile's neighbour records (its list entry came in during
+            // the previous tile) and the list entry of the tile after it;
             // every copy has landed by this tile's cp.async waits
-            if (item + gridDim.x < n_active && threadIdx.x < 10) {
-                const uint32_t tn = s_tile[nb];
-                if (threadIdx.x == 9) {
-                    cp_async<8>(&s_range[nb], &c.tile_range[tn]);
-                } else {
-                    const uint32_t ln = tn - P.tile_base;
-                    const int sx = (int)(ln % P.tiles_x) + (int)(threadIdx.x % 3) - 1;
-                    const int sy = (int)(ln / P.tiles_x) + (int)(threadIdx.x / 3) - 1;
-                    if (sx >= 0 && sy >= 0 && sx < tiles_x && sy < tiles_y)
-                        cp_async<8>(&s_infos[nb][threadIdx.x], &c.tile_info[P.tile_base + (uint32_t)(sy * tiles_x + sx)]);
-                    else
-                        s_infos[nb][threadIdx.x] = make_uint2(0xffffffffu, 0u);
-                }
+            if (item + gridDim.x < n_items && threadIdx.x < 9) {
+                const uint32_t ln = s_item[nb].x - P.tile_base;
+                const int sx = (int)(ln % P.tiles_x) + (int)(threadIdx.x % 3) - 1;
+                const int sy = (int)(ln / P.tiles_x) + (int)(threadIdx.x / 3) - 1;
+                if (sx >= 0 && sy >= 0 && sx < tiles_x && sy < tiles_y)
+                    cp_async<8>(&s_infos[nb][threadIdx.x], &c.tile_info[P.tile_base + (uint32_t)(sy * tiles_x + sx)]);
+                else
+                    s_infos[nb][threadIdx.x] = make_uint2(0xffffffffu, 0u);
             }
-            if (threadIdx.x == 10 && item + 2u * gridDim.x < n_active)
-                cp_async<4>(&s_tile[buf], listed_tile(c0, item + 2u * gridDim.x, n_heavy));
+            if (threadIdx.x == 10 && item + 2u * gridDim.x < n_items)
+                cp_async<16>(&s_item[buf], item_at(item + 2u * gridDim.x));
         }
         if (s_fail) {
             cp_async_wait_all();  // no copy may land after this tile's shared data is reused
@@ -2466,6 +2587,7 @@ __device__ __forceinline__ void g2p_tiles(const Ctx &c0, G2PShared &sh)
 template <bool SCENES, bool BODIES, bool LIQ, bool REC>
 __global__ void __launch_bounds__(G2P_THREADS, 4) k_g2p_tile(Ctx c0)
 {
+    follow();
     __shared__ G2PShared sh;
     g2p_tiles<SCENES, BODIES, LIQ, REC>(c0, sh);
 }
@@ -2589,6 +2711,7 @@ size_t substep_shared_bytes(int cap) { return std::max(p2g_shared_bytes(cap), si
 // of the default path): begin_substep for every scene.
 __global__ void k_substep_begin(Ctx c)
 {
+    follow();
     for (uint32_t s = blockIdx.x * blockDim.x + threadIdx.x; s < c.n_scenes; s += gridDim.x * blockDim.x)
         begin_substep(scene_ctx(c, s));
 }
@@ -2607,6 +2730,7 @@ __global__ void k_substep_begin(Ctx c)
 // may ask batch_stop first, which answers the same before and after.
 __global__ void k_end_batch(Ctx c0, uint32_t total, uint32_t measure_speed)
 {
+    follow();
     if (blockIdx.x == 0) {
         for (uint32_t s = threadIdx.x; s < c0.n_scenes; s += blockDim.x) {
             const Ctx cs = scene_ctx(c0, s);
@@ -2936,6 +3060,7 @@ __device__ __forceinline__ bool move_vertex(const Ctx &c, uint32_t slot, float2 
 // float64 (triangle_sample_f64).
 __global__ void __launch_bounds__(TILE_NODES) k_triangle_field(Ctx c)
 {
+    follow();
     const StepParams &P = *c.P;
     __shared__ float2 s_v0[FIELD_BODY_CHUNK], s_v1[FIELD_BODY_CHUNK], s_v2[FIELD_BODY_CHUNK];
     __shared__ float2 s_min[FIELD_BODY_CHUNK], s_max[FIELD_BODY_CHUNK];
@@ -3019,6 +3144,7 @@ __global__ void __launch_bounds__(TILE_NODES) k_triangle_field(Ctx c)
 // vertex velocities.
 __global__ void __launch_bounds__(BODY_THREADS) k_body_impulses(Ctx c)
 {
+    follow();
     const StepParams &P = *c.P;
     __shared__ int s_valid;
     __shared__ int s_box[4];
@@ -3100,6 +3226,7 @@ __global__ void __launch_bounds__(BODY_THREADS) k_body_impulses(Ctx c)
 // min(k (dt / dtRef)^2, 1); the displacement also enters the velocity.
 __global__ void k_body_bonded(Ctx c)
 {
+    follow();
     const StepParams &P = *c.P;
     const uint32_t b = blockIdx.x * blockDim.x + threadIdx.x;
     if (b >= P.n_bodies || *(volatile uint32_t *)c.status != 0u) return;
@@ -3165,6 +3292,7 @@ __global__ void k_body_bonded(Ctx c)
 // else from a scan of the other bodies here.
 __global__ void k_body_states(Ctx c)
 {
+    follow();
     const StepParams &P = *c.P;
     const uint32_t b = blockIdx.x * blockDim.x + threadIdx.x;
     if (b >= P.n_bodies || *(volatile uint32_t *)c.status != 0u) return;
@@ -3201,6 +3329,7 @@ __global__ void k_body_states(Ctx c)
 // unordered body pair of different objects, and the contact degrees.
 __global__ void k_body_pairs(Ctx c)
 {
+    follow();
     const StepParams &P = *c.P;
     const uint32_t nb = P.n_bodies;
     const uint32_t pair = blockIdx.x * blockDim.x + threadIdx.x;
@@ -3222,6 +3351,7 @@ __global__ void k_body_pairs(Ctx c)
 // larger contact degree, added to the three vertex velocities.
 __global__ void k_body_apply(Ctx c)
 {
+    follow();
     const StepParams &P = *c.P;
     const uint32_t nb = P.n_bodies;
     const uint32_t b = blockIdx.x * blockDim.x + threadIdx.x;
@@ -3284,6 +3414,7 @@ __global__ void k_body_apply(Ctx c)
 // after the body passes (G2P checks them itself when there are no bodies).
 __global__ void k_validate_cfl(Ctx c)
 {
+    follow();
     const uint32_t d = blockIdx.x * blockDim.x + threadIdx.x;
     if (d >= c.n) return;
     const Material m = c.mats[c.out.mat[d]];
@@ -3294,6 +3425,7 @@ __global__ void k_validate_cfl(Ctx c)
 // from the committed positions -> damage, broken latch.
 __global__ void k_fracture_bonds(Ctx c)
 {
+    follow();
     const StepParams &P = *c.P;
     const uint32_t bi = blockIdx.x * blockDim.x + threadIdx.x;
     if (bi >= P.n_bonds || *(volatile uint32_t *)c.status != 0u) return;
@@ -3330,6 +3462,7 @@ __global__ void k_fracture_bonds(Ctx c)
 // takes the largest damage of its bonds (CSR incidence).
 __global__ void k_fracture_damage(Ctx c)
 {
+    follow();
     const StepParams &P = *c.P;
     const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= c.n_endpoints || *(volatile uint32_t *)c.status != 0u) return;
@@ -3359,6 +3492,7 @@ __global__ void k_fracture_damage(Ctx c)
 // left them out).
 __global__ void k_body_finish(Ctx c)
 {
+    follow();
     const StepParams &P = *c.P;
     const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= c.n_tracked || *(volatile uint32_t *)c.status != 0u) return;

@@ -83,7 +83,9 @@ struct Ctx {
     // tile buckets and the per-tile partial node sums of the default P2G
     uint32_t *tile_count;
     uint2 *tile_range;       // per tile listed this substep: first bucket entry, particles
-    uint32_t *active_tiles;  // tiles holding particles this substep
+    uint4 *active_tiles;     // tiles holding particles this substep: tile, first bucket entry, particles, 0
+    uint4 *g2p_items;        // G2P's items of work, like active_tiles: those, or with `divided` a list of its own
+    uint32_t divided;        // k_tile_bucket lists the items of G2P, a tile in one or more parts
     const uint32_t *scene_chunk;  // per scene: its first CTA of k_tile_alloc, then the CTA total
     float *part;             // per tile: ACC_WORDS x RING_NODES sums, word-major
     uint2 *tile_info;        // per tile: (substep stamp of the sums, channel mask)
@@ -132,6 +134,8 @@ constexpr int SCAN_CHUNK = SCAN_THREADS * SCAN_ITEMS;
 constexpr int SCAN_TOP_THREADS = 1024;
 constexpr int ALLOC_THREADS = 256;  // k_tile_alloc: 4 tiles per thread, 1024 per CTA
 constexpr int ALLOC_ITEMS = 4;
+constexpr int BUCKET_THREADS = 1024;  // k_tile_bucket: 4 tiles and 4 slots per thread
+constexpr uint32_t BUCKET_TILES = BUCKET_THREADS * 4;
 constexpr uint32_t ALLOC_TILES = ALLOC_THREADS * ALLOC_ITEMS;
 
 // default P2G: the particles whose base node lies in one 16x8-node tile reach
@@ -149,6 +153,7 @@ constexpr uint32_t KEY_TILE_MASK = (1u << KEY_CELL_SHIFT) - 1u;
 constexpr int VOL_X = RING_X + 2;          // ring nodes and their neighbours
 constexpr int VOL_Y = RING_Y + 2;
 constexpr int G2P_THREADS = 256;
+constexpr uint32_t G2P_MAX_PARTS = 4;      // CTAs that may share a tile in G2P
 constexpr int FIELD_BODY_CHUNK = TILE_NODES;  // bodies staged per pass of k_triangle_field
 constexpr int BODY_THREADS = 64;              // k_body_impulses: one CTA per body
 constexpr uint32_t PAIR_CACHE_BODIES = 2048;  // bodies up to which pair contacts are cached
@@ -171,6 +176,8 @@ constexpr int WORK_BARRIER = 2;  // work[2]: arrivals at the substep kernel's gr
 constexpr int WORK_ABORT = 4;    // work[4]: non-zero once a barrier wait of the substep kernel ran out
 constexpr int WORK_HEAVY = 5;    // work[5], work[6]: heavy tiles listed for the substeps from buffer 0 / 1
 constexpr int WORK_CLAIM = 7;    // work[7], work[8]: tiles claimed so far by this substep's P2G / G2P (several scenes)
+constexpr int WORK_TICKET = 9;   // work[9]: CTAs of k_tile_bucket that have read the scene's counters
+constexpr int WORK_ITEMS = 10;   // work[10], work[11]: G2P items listed for the substeps from buffer 0 / 1
 constexpr int WORK_WORDS = 16;
 constexpr uint32_t HEAVY_TILE = 640;  // a tile holding more particles is listed first (it takes longest)
 constexpr int SUBSTEP_THREADS = 256;  // k_substep: one CTA shape for all four phases
@@ -184,6 +191,7 @@ __global__ void k_stable_rank(Ctx c);
 __global__ void k_tile_count(Ctx c);
 __global__ void k_tile_alloc(Ctx c);
 __global__ void k_tile_scatter(Ctx c);
+__global__ void k_tile_bucket(Ctx c);
 // SCENES: the solver holds several scenes; CAP: particles staged at once;
 // ROLES: threads per cell of a tile; LIQ: every material is water or oil; REC: the records variant (P2G reads
 // the records G2P wrote instead of preparing each particle from its state)

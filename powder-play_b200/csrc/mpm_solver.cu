@@ -124,7 +124,8 @@ struct mpm_solver {
     float4 *g_water = nullptr, *g_oil = nullptr;
     int32_t *fixed = nullptr;
     uint32_t *tile_stamp = nullptr;
-    uint32_t *tile_count = nullptr, *active_tiles = nullptr;
+    uint32_t *tile_count = nullptr;
+    uint4 *active_tiles = nullptr;
     uint2 *tile_range = nullptr;
     uint32_t *scene_chunk = nullptr;  // per scene: first CTA of k_tile_alloc, then the total
     uint32_t alloc_ctas = 1;
@@ -225,6 +226,27 @@ bool uses_records(const mpm_solver *s)
     return false;
 }
 
+// Enqueues a kernel of the substep chain.
+template <class... Args>
+void launch(mpm_solver *s, void (*kernel)(Args...), dim3 grid, dim3 block, size_t shared, Args... args)
+{
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = shared;
+    cfg.stream = s->stream;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    cudaLaunchKernelEx(&cfg, kernel, args...);
+}
+
+// Whether k_tile_bucket buckets the particles (else k_tile_alloc and
+// k_tile_scatter): one scene whose tiles each of its CTAs can scan at once.
+bool buckets_at_once(const mpm_solver *s) { return s->n_scenes == 1 && s->scenes[0].tiles <= BUCKET_TILES && !s->fused; }
+
 Ctx make_ctx(mpm_solver *s, int parity)
 {
     Ctx c{};
@@ -266,6 +288,10 @@ Ctx make_ctx(mpm_solver *s, int parity)
     c.tile_range = s->tile_range;
     c.scene_chunk = s->scene_chunk;
     c.active_tiles = s->active_tiles;
+    // about an item of G2P per SM at most (48,000 particles: no gain); a body's
+    // impulses are stored by one CTA per tile
+    c.divided = buckets_at_once(s) && s->n <= G2P_THREADS * s->sms && s->n_tracked == 0 && s->n_bodies == 0 ? 1u : 0u;
+    c.g2p_items = c.divided ? s->active_tiles + s->n_tiles_total : s->active_tiles;
     c.part = s->part;
     c.tile_info = s->tile_info;
     const bool rec = s->gather() && uses_records(s);
@@ -301,11 +327,11 @@ constexpr unsigned PARTICLE_THREADS = 256;
 // Kernel slots of the profiled substep (mpm_profile_substeps).
 enum KernelSlot {
     K_TILE_COUNT, K_TILE_ALLOC, K_TILE_SCATTER, K_P2G_GATHER, K_G2P_TILE, K_PREPARE_SCATTER,
-    K_FIXED_DECODE, K_GRID_UPDATE, K_G2P, K_SUBSTEP_BEGIN, K_END_BATCH, K_SUBSTEP, K_SLOTS
+    K_FIXED_DECODE, K_GRID_UPDATE, K_G2P, K_SUBSTEP_BEGIN, K_END_BATCH, K_SUBSTEP, K_TILE_BUCKET, K_SLOTS
 };
 const char *const KERNEL_NAMES[K_SLOTS] = {
     "k_tile_count", "k_tile_alloc", "k_tile_scatter", "k_p2g_gather", "k_g2p_tile", "k_prepare_scatter",
-    "k_fixed_decode", "k_grid_update", "k_g2p", "k_substep_begin", "k_end_batch", "k_substep"};
+    "k_fixed_decode", "k_grid_update", "k_g2p", "k_substep_begin", "k_end_batch", "k_substep", "k_tile_bucket"};
 
 // When set, an event is recorded after every kernel launch so that the
 // kernels of a substep can be timed one by one.  The profiled substeps are
@@ -340,7 +366,7 @@ inline void mark(int slot)
 void enqueue_tile_count(mpm_solver *s, const Ctx &c)
 {
     cudaMemsetAsync(s->tile_count, 0, (size_t)s->n_tiles_total * sizeof(uint32_t), s->stream);
-    k_tile_count<<<blocks_for(s->n, PARTICLE_THREADS), PARTICLE_THREADS, 0, s->stream>>>(c);
+    launch(s, k_tile_count, dim3(blocks_for(s->n, PARTICLE_THREADS)), dim3(PARTICLE_THREADS), 0, c);
     mark(K_TILE_COUNT);
 }
 
@@ -366,20 +392,20 @@ void enqueue_bodies(mpm_solver *s, const Ctx &c)
     const uint32_t nb = s->n_bodies;
     if (nb) {
         const unsigned bb = blocks_for(nb, 64);
-        k_body_impulses<<<std::min(nb, 1024u), BODY_THREADS, 0, s->stream>>>(c);
-        k_body_bonded<<<bb, 64, 0, s->stream>>>(c);
-        k_body_states<<<bb, 64, 0, s->stream>>>(c);
-        if (s->pair_cache) k_body_pairs<<<blocks_for(nb * nb, 256), 256, 0, s->stream>>>(c);
-        k_body_apply<<<bb, 64, 0, s->stream>>>(c);
+        launch(s, k_body_impulses, dim3(std::min(nb, 1024u)), dim3(BODY_THREADS), 0, c);
+        launch(s, k_body_bonded, dim3(bb), dim3(64), 0, c);
+        launch(s, k_body_states, dim3(bb), dim3(64), 0, c);
+        if (s->pair_cache) launch(s, k_body_pairs, dim3(blocks_for(nb * nb, 256)), dim3(256), 0, c);
+        launch(s, k_body_apply, dim3(bb), dim3(64), 0, c);
         // captured graphs serve batches with and without a CFL guard: the
         // kernel reads the batch's flag from the device parameters
-        k_validate_cfl<<<blocks_for(s->n, PARTICLE_THREADS), PARTICLE_THREADS, 0, s->stream>>>(c);
+        launch(s, k_validate_cfl, dim3(blocks_for(s->n, PARTICLE_THREADS)), dim3(PARTICLE_THREADS), 0, c);
     }
     if (s->n_bonds) {
-        k_fracture_bonds<<<blocks_for(s->n_bonds, 64), 64, 0, s->stream>>>(c);
-        if (s->n_endpoints) k_fracture_damage<<<blocks_for(s->n_endpoints, 64), 64, 0, s->stream>>>(c);
+        launch(s, k_fracture_bonds, dim3(blocks_for(s->n_bonds, 64)), dim3(64), 0, c);
+        if (s->n_endpoints) launch(s, k_fracture_damage, dim3(blocks_for(s->n_endpoints, 64)), dim3(64), 0, c);
     }
-    if (s->gather() && s->n_tracked) k_body_finish<<<blocks_for(s->n_tracked, 64), 64, 0, s->stream>>>(c);
+    if (s->gather() && s->n_tracked) launch(s, k_body_finish, dim3(blocks_for(s->n_tracked, 64)), dim3(64), 0, c);
 }
 
 // The k_substep instantiation for the scene count, stage capacity and
@@ -500,15 +526,15 @@ template <bool REC>
 void launch_g2p(mpm_solver *s, const Ctx &c, bool liq)
 {
     if (s->n_scenes > 1 && liq)
-        k_g2p_tile<true, false, true, REC><<<s->g2p_ctas, G2P_THREADS, 0, s->stream>>>(c);
+        launch(s, k_g2p_tile<true, false, true, REC>, dim3(s->g2p_ctas), dim3(G2P_THREADS), 0, c);
     else if (s->n_scenes > 1)
-        k_g2p_tile<true, false, false, REC><<<s->g2p_ctas, G2P_THREADS, 0, s->stream>>>(c);
+        launch(s, k_g2p_tile<true, false, false, REC>, dim3(s->g2p_ctas), dim3(G2P_THREADS), 0, c);
     else if (s->n_tracked > 0)
-        k_g2p_tile<false, true, false, REC><<<s->g2p_ctas, G2P_THREADS, 0, s->stream>>>(c);
+        launch(s, k_g2p_tile<false, true, false, REC>, dim3(s->g2p_ctas), dim3(G2P_THREADS), 0, c);
     else if (liq)
-        k_g2p_tile<false, false, true, REC><<<s->g2p_ctas, G2P_THREADS, 0, s->stream>>>(c);
+        launch(s, k_g2p_tile<false, false, true, REC>, dim3(s->g2p_ctas), dim3(G2P_THREADS), 0, c);
     else
-        k_g2p_tile<false, false, false, REC><<<s->g2p_ctas, G2P_THREADS, 0, s->stream>>>(c);
+        launch(s, k_g2p_tile<false, false, false, REC>, dim3(s->g2p_ctas), dim3(G2P_THREADS), 0, c);
 }
 
 // One full substep from buffer `parity` into 1 - parity.
@@ -522,18 +548,23 @@ void enqueue_substep(mpm_solver *s, int parity)
         if (e != cudaSuccess && g_recorder && g_recorder->error == cudaSuccess) g_recorder->error = e;
         mark(K_SUBSTEP);
     } else if (s->gather()) {
-        k_tile_alloc<<<s->alloc_ctas, ALLOC_THREADS, 0, s->stream>>>(c);
-        mark(K_TILE_ALLOC);
-        k_tile_scatter<<<blocks_for((s->n + 3) / 4, PARTICLE_THREADS), PARTICLE_THREADS, 0, s->stream>>>(c);
-        mark(K_TILE_SCATTER);
+        if (buckets_at_once(s)) {
+            launch(s, k_tile_bucket, dim3(blocks_for((s->n + 3) / 4, BUCKET_THREADS)), dim3(BUCKET_THREADS), 0, c);
+            mark(K_TILE_BUCKET);
+        } else {
+            launch(s, k_tile_alloc, dim3(s->alloc_ctas), dim3(ALLOC_THREADS), 0, c);
+            mark(K_TILE_ALLOC);
+            launch(s, k_tile_scatter, dim3(blocks_for((s->n + 3) / 4, PARTICLE_THREADS)), dim3(PARTICLE_THREADS), 0, c);
+            mark(K_TILE_SCATTER);
+        }
         {
-            void *args[] = {const_cast<Ctx *>(&c)};
-            cudaLaunchKernel(p2g_kernel(s->n_scenes > 1, s->stage_cap, p2g_roles(s), runs_liquid(s), uses_records(s)),
-                             dim3(s->p2g_ctas), dim3(p2g_roles(s) * TILE_CELLS), args,
-                             p2g_shared_bytes(s->stage_cap), s->stream);
+            using Kernel = void (*)(Ctx);
+            launch(s, reinterpret_cast<Kernel>(const_cast<void *>(p2g_kernel(s->n_scenes > 1, s->stage_cap, p2g_roles(s),
+                                                                             runs_liquid(s), uses_records(s)))),
+                   dim3(s->p2g_ctas), dim3(p2g_roles(s) * TILE_CELLS), p2g_shared_bytes(s->stage_cap), c);
         }
         mark(K_P2G_GATHER);
-        if (s->n_bodies) k_triangle_field<<<tiles, TILE_NODES, 0, s->stream>>>(c);
+        if (s->n_bodies) launch(s, k_triangle_field, tiles, dim3(TILE_NODES), 0, c);
         const bool liq = runs_liquid(s);
         if (uses_records(s))
             launch_g2p<true>(s, c, liq);
@@ -541,16 +572,16 @@ void enqueue_substep(mpm_solver *s, int parity)
             launch_g2p<false>(s, c, liq);
         mark(K_G2P_TILE);
     } else {
-        k_substep_begin<<<blocks_for(s->n_scenes, PARTICLE_THREADS), PARTICLE_THREADS, 0, s->stream>>>(c);
+        launch(s, k_substep_begin, dim3(blocks_for(s->n_scenes, PARTICLE_THREADS)), dim3(PARTICLE_THREADS), 0, c);
         mark(K_SUBSTEP_BEGIN);
-        k_prepare_scatter<<<pb, PARTICLE_THREADS, 0, s->stream>>>(c);
+        launch(s, k_prepare_scatter, dim3(pb), dim3(PARTICLE_THREADS), 0, c);
         mark(K_PREPARE_SCATTER);
-        k_fixed_decode<<<tiles, TILE_NODES, 0, s->stream>>>(c);
+        launch(s, k_fixed_decode, tiles, dim3(TILE_NODES), 0, c);
         mark(K_FIXED_DECODE);
-        if (s->n_bodies) k_triangle_field<<<tiles, TILE_NODES, 0, s->stream>>>(c);
-        k_grid_update<<<tiles, TILE_NODES, 0, s->stream>>>(c);
+        if (s->n_bodies) launch(s, k_triangle_field, tiles, dim3(TILE_NODES), 0, c);
+        launch(s, k_grid_update, tiles, dim3(TILE_NODES), 0, c);
         mark(K_GRID_UPDATE);
-        k_g2p<<<pb, PARTICLE_THREADS, 0, s->stream>>>(c);
+        launch(s, k_g2p, dim3(pb), dim3(PARTICLE_THREADS), 0, c);
         mark(K_G2P);
     }
     enqueue_bodies(s, c);
@@ -562,7 +593,7 @@ void enqueue_end_batch(mpm_solver *s, int parity, uint32_t total, bool measure_s
     const Ctx c = make_ctx(s, 1 - parity);  // out: the buffer the batch ends in
     const unsigned ctas = s->n_scenes == 1 ? blocks_for(s->n, END_BATCH_THREADS * END_BATCH_ITEMS)
                                            : std::min(blocks_for(s->n, END_BATCH_THREADS), 1184u);
-    k_end_batch<<<ctas, END_BATCH_THREADS, 0, s->stream>>>(c, total, measure_speed ? 1u : 0u);
+    launch(s, k_end_batch, dim3(ctas), dim3(END_BATCH_THREADS), 0, c, total, measure_speed ? 1u : 0u);
     mark(K_END_BATCH);
 }
 
@@ -1079,7 +1110,7 @@ int create_impl(const mpm_config *configs, uint32_t n_scenes, const uint32_t *co
             return fail(set_error(MPM_ERR_CUDA, "scene table upload failed"));
     }
     if (c.p2g_mode == MPM_P2G_GATHER) {
-        ALLOC(s->active_tiles, n_tiles);
+        ALLOC(s->active_tiles, n_tiles * (1 + G2P_MAX_PARTS));
         ALLOC(s->part, n_tiles * ACC_WORDS * RING_NODES);
         ALLOC(s->tile_info, n_tiles);
         s->rec_state = reinterpret_cast<float4 *>(s->slab);
@@ -1098,7 +1129,7 @@ int create_impl(const mpm_config *configs, uint32_t n_scenes, const uint32_t *co
             return fail(set_error(MPM_ERR_CUDA, "occupancy query failed"));
         s->sms = (unsigned)sms;
         s->p2g_ctas = (unsigned)std::max<size_t>(1, std::min<size_t>(n_tiles, (size_t)sms * std::max(1, per_sm_p2g)));
-        s->g2p_ctas = (unsigned)std::max<size_t>(1, std::min<size_t>(n_tiles, (size_t)sms * std::max(1, per_sm_g2p)));
+        s->g2p_ctas = (unsigned)std::max<size_t>(1, std::min<size_t>(n_tiles * G2P_MAX_PARTS, (size_t)sms * std::max(1, per_sm_g2p)));
         s->substep_max_ctas = (unsigned)std::max(1, sms * per_sm_substep);
         s->substep_ctas = s->substep_max_ctas;
     }
@@ -1209,7 +1240,7 @@ int profile_run(mpm_solver *s, uint32_t step_count, bool guarded, double *kernel
     const Ctx c0 = make_ctx(s, s->cur);
     const int start_parity = s->cur;
     CUDA_TRY(cudaStreamBeginCapture(s->stream, cudaStreamCaptureModeThreadLocal));
-    k_begin_batch<<<blocks_for(s->n_scenes, PARTICLE_THREADS), PARTICLE_THREADS, 0, s->stream>>>(c0, guarded ? 1u : 0u);
+    launch(s, k_begin_batch, dim3(blocks_for(s->n_scenes, PARTICLE_THREADS)), dim3(PARTICLE_THREADS), 0, c0, guarded ? 1u : 0u);
     rec.mark(-1);
     g_recorder = &rec;
     if (s->gather() && s->n > 0) enqueue_tile_count(s, c0);
@@ -1250,7 +1281,7 @@ int timed_run(mpm_solver *s, uint32_t step_count, bool guarded, double *ms)
 {
     const Ctx c0 = make_ctx(s, s->cur);
     CUDA_TRY(cudaStreamBeginCapture(s->stream, cudaStreamCaptureModeThreadLocal));
-    k_begin_batch<<<blocks_for(s->n_scenes, PARTICLE_THREADS), PARTICLE_THREADS, 0, s->stream>>>(c0, guarded ? 1u : 0u);
+    launch(s, k_begin_batch, dim3(blocks_for(s->n_scenes, PARTICLE_THREADS)), dim3(PARTICLE_THREADS), 0, c0, guarded ? 1u : 0u);
     if (s->gather() && s->n > 0) enqueue_tile_count(s, c0);
     int parity = s->cur;
     for (uint32_t k = 0; k < step_count; ++k) {
@@ -1420,7 +1451,7 @@ cudaError_t capture_batch(mpm_solver *s, uint32_t step_count, int parity, bool g
     if (e == cudaSuccess) e = cudaEventRecordWithFlags(s->batch_start, s->stream, cudaEventRecordExternal);
     if (e != cudaSuccess) return e;
     const Ctx c0 = make_ctx(s, parity);
-    k_begin_batch<<<blocks_for(s->n_scenes, PARTICLE_THREADS), PARTICLE_THREADS, 0, s->stream>>>(c0, guarded ? 1u : 0u);
+    launch(s, k_begin_batch, dim3(blocks_for(s->n_scenes, PARTICLE_THREADS)), dim3(PARTICLE_THREADS), 0, c0, guarded ? 1u : 0u);
     if (s->gather()) enqueue_tile_count(s, c0);
     int p = parity;
     for (uint32_t k = 0; k < step_count; ++k) {
@@ -1480,7 +1511,7 @@ int run_batch(mpm_solver *s, uint32_t step_count, bool guarded)
     if (rc != MPM_OK) return rc;
     const Ctx c0 = make_ctx(s, s->cur);
     CUDA_TRY(cudaEventRecord(s->batch_start, s->stream));
-    k_begin_batch<<<blocks_for(s->n_scenes, PARTICLE_THREADS), PARTICLE_THREADS, 0, s->stream>>>(c0, guarded ? 1u : 0u);
+    launch(s, k_begin_batch, dim3(blocks_for(s->n_scenes, PARTICLE_THREADS)), dim3(PARTICLE_THREADS), 0, c0, guarded ? 1u : 0u);
     if (s->gather() && s->n > 0) enqueue_tile_count(s, c0);
     CUDA_TRY(cudaGetLastError());
     if (s->n > 0) {

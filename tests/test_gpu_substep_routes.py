@@ -2,7 +2,9 @@
 one-launch substep, which takes the same arithmetic through one route at all
 sizes (two threads per cell in P2G; tile allocation and bucketing of their
 own).  One scene steps with two threads per cell up to 640 particles per SM and
-with one above."""
+with one above; its tiles are bucketed by one kernel up to 4,096 of them and by
+two above; and G2P takes a tile in up to four parts while there are at most 256
+particles per SM."""
 import numpy as np
 import pytest
 
@@ -38,6 +40,11 @@ def _scene(n, cells_x, cells_y, spacing):
     (257, 17, 33, 5.0),
     (640 * SMS, 400, 400, 5.0),      # the last size with two threads per cell
     (640 * SMS + 1, 400, 400, 5.0),  # and the first with one
+    (256 * SMS, 300, 250, 5.0),      # the last size whose tiles G2P divides
+    (256 * SMS + 1, 300, 250, 5.0),
+    (3_000, 17, 33, 3.0),            # more items than tiles
+    (30_001, 1021, 509, 5.0),        # 4,096 tiles: bucketed by one kernel
+    (30_001, 1021, 510, 5.0),        # 4,160
     (60_001, 120, 130, 2.5),         # 16 particles per cell: every tile above one stage
 ])
 def test_every_route_gives_the_one_launch_bits(n, cells_x, cells_y, spacing):
