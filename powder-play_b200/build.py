@@ -12,7 +12,7 @@ HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 OUTPUT = os.path.join(HERE, "libmpm_b200.so")
 SOURCES = ["mpm_kernels.cu", "mpm_solver.cu", "mpm_static_sort.cu", "mpm_adjoint.cu", "mpm_records.cu"]
-HEADERS = ["mpm_device.cuh", "mpm_kernels.cuh", "mpm_records.cuh"]
+HEADERS = ["mpm_device.cuh", "mpm_kernels.cuh", "mpm_launch.cuh", "mpm_records.cuh"]
 
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a",

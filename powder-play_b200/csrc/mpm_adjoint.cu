@@ -21,12 +21,14 @@
 // rotation by atan2(F10 - F01, F00 + F11), which is what both the forward and
 // the adjoint use.
 //
-// Per backward segment of K substeps: the segment's start state is restored
-// from its checkpoint, the K substeps are recomputed keeping each substep's
-// input state and grid sums, then each substep is reversed by two kernels: the
-// G2P adjoint (scatters the node-velocity adjoints) and the fused grid + P2G
-// adjoint (gathers them back to the particle and adds the parameter
-// gradients).
+// A forward substep is two kernels: the grid update, and G2P with the P2G of
+// the next substep (the particle's new state is in registers there).  Per
+// backward segment of K substeps: the K substeps are recomputed from the
+// segment's checkpoint, keeping each substep's input state and grid sums (the
+// last segment's are kept by the forward pass), then each substep is reversed by
+// four: the grid update again, the G2P adjoint (scatters the node-velocity
+// adjoints), the grid adjoint, and the P2G adjoint (gathers them back to the
+// particle and adds the parameter gradients).
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -40,6 +42,8 @@
 
 #include "../../include/mpm_b200.h"
 #include "mpm_device.cuh"
+#include "mpm_launch.cuh"
+#include "mpm_records.cuh"
 
 namespace mpm {
 int host_error(int code, const char *message);
@@ -51,6 +55,7 @@ using namespace mpm;
 namespace {
 
 constexpr unsigned ADJ_THREADS = 256;
+
 
 // Per-scene constants; tait, lambda_s and mu_s are the differentiated
 // material parameters.
@@ -70,8 +75,7 @@ struct AdjState {
 
 struct AdjCtx {
     const AdjScene *scenes;
-    const uint32_t *scene_of;  // per particle
-    const uint32_t *liquid;    // per particle: 1 Tait water, 0 fixed-corotated solid
+    const uint32_t *tag;       // per particle: scene << 1 | 1 for Tait water, 0 for a fixed-corotated solid
     const float *vol;          // per particle
     uint32_t n;
     uint32_t *status;
@@ -89,10 +93,10 @@ struct AdjCtx {
     double *param_grad;    // per scene: tait, lambda_s, mu_s
     const float2 *target;  // per particle
     double *loss;          // per scene
-    uint8_t *mark_out;     // per tile: marked when a new position's stencil reaches it (k_adj_g2p), or NULL
+    uint8_t *mark_out;     // per tile, solid and water: set when a position whose P2G is scattered reaches it, or NULL
 };
 
-constexpr int ADJ_TILE = 16;  // nodes per side of a clearing tile
+constexpr int ADJ_TILE = 16;  // nodes per side of a tile of marks
 
 constexpr uint32_t ADJ_ERR_STENCIL = 1u, ADJ_ERR_NONFINITE = 2u, ADJ_ERR_DETERMINANT = 4u;
 
@@ -363,33 +367,33 @@ __device__ __forceinline__ float4 project_liquid(float4 T)
 
 }  // namespace
 
-// Marks the clearing tiles that the stencil with base (bx, by) reaches (its
-// corner nodes lie in at most four).  Lanes of a warp storing to the same
-// mark byte in one instruction make one memory transaction.
-__device__ __forceinline__ void mark_tiles(uint8_t *mark, const AdjScene &S, int bx, int by)
+// Marks the tiles that the stencil with base (bx, by) reaches (its corner
+// nodes lie in at most four), a byte for solid particles and one for water.  Lanes
+// of a warp storing to the same mark byte in one instruction make one memory
+// transaction.
+__device__ __forceinline__ void mark_tiles(uint8_t *mark, const AdjScene &S, bool liquid, int bx, int by)
 {
     const uint32_t x0 = (uint32_t)(bx + 1) / ADJ_TILE, x1 = (uint32_t)(bx + 3) / ADJ_TILE;
     const uint32_t y0 = (uint32_t)(by + 1) / ADJ_TILE, y1 = (uint32_t)(by + 3) / ADJ_TILE;
-    uint8_t *row0 = mark + S.tile_base + y0 * S.tiles_x, *row1 = mark + S.tile_base + y1 * S.tiles_x;
-    row0[x0] = 1u;
-    if (x1 != x0) row0[x1] = 1u;
+    mark += 2u * S.tile_base + (liquid ? 1u : 0u);
+    uint8_t *row0 = mark + 2u * y0 * S.tiles_x, *row1 = mark + 2u * y1 * S.tiles_x;
+    row0[2u * x0] = 1u;
+    if (x1 != x0) row0[2u * x1] = 1u;
     if (y1 != y0) {
-        row1[x0] = 1u;
-        if (x1 != x0) row1[x1] = 1u;
+        row1[2u * x0] = 1u;
+        if (x1 != x0) row1[2u * x1] = 1u;
     }
 }
 
 // ------------------------------------------------------------- kernels ----
 
-__global__ void __launch_bounds__(ADJ_THREADS) k_adj_p2g(AdjCtx c)
+// The P2G of one particle: adds to the node sums and marks the tiles its
+// stencil reaches (unless mark_out is NULL), or raises a status.
+__device__ __forceinline__ void p2g_particle(const AdjCtx &c, const AdjScene &S, bool liquid, float2 x, float2 v, float4 C,
+                                             float4 F, float vol)
 {
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= c.n) return;
-    const AdjScene &S = c.scenes[c.scene_of[i]];
-    const bool liquid = c.liquid[i] != 0u;
-    const float2 x = c.in.x[i], v = c.in.v[i];
     Prepared p;
-    if (!adj_prepare(S, liquid, c.vol[i], c.in.C[i], c.in.F[i], p)) {
+    if (!adj_prepare(S, liquid, vol, C, F, p)) {
         adj_fail(c, ADJ_ERR_DETERMINANT);
         return;
     }
@@ -398,7 +402,8 @@ __global__ void __launch_bounds__(ADJ_THREADS) k_adj_p2g(AdjCtx c)
         adj_fail(c, ADJ_ERR_STENCIL);
         return;
     }
-    float4 *sums = liquid ? c.sum_w : c.sum_s;
+    if (c.mark_out) mark_tiles(c.mark_out, S, liquid, st.bx, st.by);
+    float4 *sums = (liquid ? c.sum_w : c.sum_s) + adj_node(S, st.bx, st.by);
 #pragma unroll
     for (int oy = 0; oy < 3; ++oy) {
         const float dpy = ((float)oy - st.fy) * S.dx;
@@ -408,20 +413,40 @@ __global__ void __launch_bounds__(ADJ_THREADS) k_adj_p2g(AdjCtx c)
             const float dpx = ((float)ox - st.fx) * S.dx;
             const float qx = p.m * v.x + p.A.x * dpx + p.A.y * dpy;
             const float qy = p.m * v.y + p.A.z * dpx + p.A.w * dpy;
-            atomicAdd(&sums[adj_node(S, st.bx + ox, st.by + oy)],
+            atomicAdd(sums + (uint32_t)oy * S.node_w + ox,
                       make_float4(w * p.m, w * qx, w * qy, liquid ? w * p.vliq : 0.f));
         }
     }
 }
 
-__global__ void __launch_bounds__(ADJ_THREADS) k_adj_g2p(AdjCtx c)
+// P2G of the states in c.in (the first substep of a run; the others' comes
+// with the G2P before them).
+__global__ void __launch_bounds__(ADJ_THREADS) k_adj_p2g(AdjCtx c)
 {
+    follow();
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= c.n) return;
-    const AdjScene &S = c.scenes[c.scene_of[i]];
-    const bool liquid = c.liquid[i] != 0u;
+    const uint32_t tag = c.tag[i];
+    p2g_particle(c, c.scenes[tag >> 1], (tag & 1u) != 0u, c.in.x[i], c.in.v[i], c.in.C[i], c.in.F[i], c.vol[i]);
+}
+
+// G2P of one substep, and with P2G the P2G of the next from the new state.
+// Latency-bound (the gathered node velocities and the particle's own words from
+// L2, issue active 40 % of cycles; the atomics use 22 % of L2's rate): 64 registers
+// for 32 warps per SM, 56.6 us at 24 warps -> 52.3 us per million particles, where
+// G2P and P2G as two kernels took 31 + 37 us and a launch more.
+template <bool P2G>
+__global__ void __launch_bounds__(ADJ_THREADS, 4) k_adj_g2p(AdjCtx c)
+{
+    follow();
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= c.n) return;
+    const uint32_t tag = c.tag[i];
+    const AdjScene &S = c.scenes[tag >> 1];
+    const bool liquid = (tag & 1u) != 0u;
     const float2 x = c.in.x[i];
     const float4 F0 = c.in.F[i];
+    const float vol = P2G ? c.vol[i] : 0.0f;
     AdjStencil st;
     G2pFwd g;
     if (!adj_stencil(S, x, st) || !g2p_forward(c, S, liquid, st, x, F0, g)) {
@@ -431,115 +456,96 @@ __global__ void __launch_bounds__(ADJ_THREADS) k_adj_g2p(AdjCtx c)
     const float4 Fn = liquid ? project_liquid(g.trial) : g.trial;
     const float2 bx = confine_axis(g.xn.x, g.vp.x, S.domain_w);
     const float2 by = confine_axis(g.xn.y, g.vp.y, S.domain_h);
-    if (c.mark_out) {
-        AdjStencil next;
-        if (adj_stencil(S, make_float2(bx.x, by.x), next)) mark_tiles(c.mark_out, S, next.bx, next.by);
-    }
-    c.out.x[i] = make_float2(bx.x, by.x);
-    c.out.v[i] = make_float2(bx.y, by.y);
+    const float2 xn = make_float2(bx.x, by.x), vn = make_float2(bx.y, by.y);
+    c.out.x[i] = xn;
+    c.out.v[i] = vn;
     c.out.C[i] = g.Cn;
     c.out.F[i] = Fn;
+    if constexpr (P2G) p2g_particle(c, S, liquid, xn, vn, g.Cn, Fn, vol);
 }
 
-// Loss sum |x - target|^2 per scene (one atomic per warp whose particles
-// share a scene) and its adjoint seeds.
-// Marks the clearing tiles the stencils of the particles in c.in reach (the
-// first substep's; later substeps' marks come from k_adj_g2p).
-__global__ void __launch_bounds__(ADJ_THREADS) k_adj_mark(AdjCtx c, uint8_t *mark)
+// The kernels over the grid take a tile of 16 x 16 nodes at a time, one node
+// per thread, and leave what no stencil of the substep reaches (`mark`, set by
+// the P2G, for solid and water) as it is: every node a substep adds to or reads
+// lies in a marked tile, and the rest of the grid keeps stale values that no
+// stencil reads.  The tiles are dealt to the CTAs one by one (marked ones lie
+// together), a CTA reads the marks of its tiles together and then visits the
+// marked ones: visit(scene, node, x, y, solid, water).  No list of the marked
+// tiles is built and no node cleared ahead of a substep: the grid update leaves the
+// sums at zero.  64 scenes of 16,384 particles, 200 substeps forward and backward:
+// 8 + 7 launches per substep -> 2 + 6, 73.9 -> 55.6 ms; one scene of 1,024, 40
+// substeps: 2.08 -> 0.93 ms.
+template <class Visit>
+__device__ __forceinline__ void for_marked_nodes(const AdjCtx &c, const uint32_t *tile_scene, const uint8_t *mark,
+                                                 uint32_t n_tiles, const Visit &visit)
 {
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= c.n) return;
-    const AdjScene &S = c.scenes[c.scene_of[i]];
-    AdjStencil st;
-    if (adj_stencil(S, c.in.x[i], st)) mark_tiles(mark, S, st.bx, st.by);
-}
-
-constexpr int COMPACT_THREADS = 256;
-
-// Appends the marked tiles of one substep to its list (list[0], zeroed before,
-// counts them; list[1 ..] holds them in no particular order: each tile is
-// cleared and updated on its own).  One tile per thread, one atomic per warp.
-__global__ void __launch_bounds__(COMPACT_THREADS) k_adj_compact(const uint8_t *mark, uint32_t n_tiles, uint32_t *list)
-{
-    const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
-    const bool marked = t < n_tiles && mark[t] != 0u;
-    const unsigned ballot = __ballot_sync(0xffffffffu, marked);
-    if (!ballot) return;
-    const uint32_t lane = threadIdx.x & 31u;
-    uint32_t base = 0;
-    if (lane == 0u) base = atomicAdd(list, (uint32_t)__popc(ballot));
-    base = __shfl_sync(0xffffffffu, base, 0);
-    if (marked) list[1 + base + __popc(ballot & ((1u << lane) - 1u))] = t;
-}
-
-// Zeroes the nodes of the listed (marked) tiles in up to three node arrays
-// (NULL: skipped), one tile per CTA iteration and one node per thread: every
-// node a substep adds to or reads lies in a tile its particles mark.  The rest
-// of the grid keeps stale values that no stencil reads.  tile_scene gives each
-// tile's scene; list[0] counts the tiles in list[1 ..].
-__global__ void __launch_bounds__(ADJ_TILE * ADJ_TILE) k_adj_clear(const AdjScene *scenes, const uint32_t *tile_scene,
-                                                                   const uint32_t *list, float4 *a, float4 *b, float2 *c2)
-{
-    const uint32_t count = list[0];
-    for (uint32_t i = blockIdx.x; i < count; i += gridDim.x) {
-        const uint32_t t = list[1 + i];
-        const AdjScene &S = scenes[tile_scene[t]];
-        const uint32_t local = t - S.tile_base;
-        const uint32_t hx = (local % S.tiles_x) * ADJ_TILE + threadIdx.x % ADJ_TILE;
-        const uint32_t hy = (local / S.tiles_x) * ADJ_TILE + threadIdx.x / ADJ_TILE;
-        if (hx >= S.node_w || hy >= S.cells_y + 3u) continue;
-        const uint32_t n = S.node_base + hy * S.node_w + hx;
-        if (a) a[n] = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (b) b[n] = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (c2) c2[n] = make_float2(0.f, 0.f);
+    __shared__ uint32_t s_tile[ADJ_THREADS], s_count;
+    for (uint32_t first = blockIdx.x; first < n_tiles; first += gridDim.x * ADJ_THREADS) {
+        __syncthreads();
+        if (threadIdx.x == 0) s_count = 0u;
+        __syncthreads();
+        const uint64_t t = first + (uint64_t)threadIdx.x * gridDim.x;
+        if (t < n_tiles) {
+            const uint32_t both = reinterpret_cast<const uint16_t *>(mark)[t];  // 1: solid, 0x100: water
+            if (both != 0u) s_tile[atomicAdd(&s_count, 1u)] = (uint32_t)t << 2 | (both & 1u) | (both >> 7 & 2u);
+        }
+        __syncthreads();
+        const uint32_t count = s_count;
+        for (uint32_t k = 0; k < count; ++k) {
+            const uint32_t entry = s_tile[k], tile = entry >> 2;
+            const AdjScene &S = c.scenes[tile_scene[tile]];
+            const uint32_t local = tile - S.tile_base;
+            const uint32_t hx = (local % S.tiles_x) * ADJ_TILE + threadIdx.x % ADJ_TILE;
+            const uint32_t hy = (local / S.tiles_x) * ADJ_TILE + threadIdx.x / ADJ_TILE;
+            if (hx < S.node_w && hy < S.cells_y + 3u)
+                visit(S, S.node_base + hy * S.node_w + hx, (int)hx - 1, (int)hy - 1, (entry & 1u) != 0u, (entry & 2u) != 0u);
+        }
     }
 }
 
-// The grid update of the marked tiles' nodes (finishGridVelocity with the
-// wall factors, node_velocity_adj): each node's velocity from its sums, once
-// per node, for the G2P kernels; the water record also carries the node's
-// liquid mass and volume.  One tile per CTA iteration, one node per thread.
-__global__ void __launch_bounds__(ADJ_TILE * ADJ_TILE) k_adj_grid_fwd(AdjCtx c, const uint32_t *tile_scene,
-                                                                      const uint32_t *list)
+// The grid update (finishGridVelocity with the wall factors,
+// node_velocity_adj): each node's velocity from its sums, for the G2P kernels;
+// the water record also carries the node's liquid mass and volume.  ZERO: the
+// sums are scratch; they are kept in tape_s / tape_w (unless NULL) and zeroed
+// for the next P2G.  Else the sums are a kept substep's, and the node adjoints
+// are zeroed for the G2P adjoint.
+template <bool ZERO>
+__global__ void __launch_bounds__(ADJ_THREADS) k_adj_grid_fwd(AdjCtx c, const uint32_t *tile_scene, const uint8_t *mark,
+                                                              uint32_t n_tiles, float4 *tape_s, float4 *tape_w)
 {
-    const uint32_t count = list[0];
-    for (uint32_t i = blockIdx.x; i < count; i += gridDim.x) {
-        const uint32_t t = list[1 + i];
-        const AdjScene &S = c.scenes[tile_scene[t]];
-        const uint32_t local = t - S.tile_base;
-        const uint32_t hx = (local % S.tiles_x) * ADJ_TILE + threadIdx.x % ADJ_TILE;
-        const uint32_t hy = (local / S.tiles_x) * ADJ_TILE + threadIdx.x / ADJ_TILE;
-        if (hx >= S.node_w || hy >= S.cells_y + 3u) continue;
-        const uint32_t n = S.node_base + hy * S.node_w + hx;
-        const int ix = (int)hx - 1, iy = (int)hy - 1;
+    follow();
+    const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+    for_marked_nodes(c, tile_scene, mark, n_tiles, [&](const AdjScene &S, uint32_t n, int ix, int iy, bool solid, bool water) {
+        float4 s, w;
+        if (solid) s = c.sum_s[n];
+        if (water) w = c.sum_w[n];
         float2 D;
-        c.gv_s[n] = node_velocity_adj(S, c.sum_s[n], ix, iy, D);
-        const float4 w = c.sum_w[n];
-        const float2 u = node_velocity_adj(S, w, ix, iy, D);
-        c.gv_w[n] = make_float4(u.x, u.y, w.x, w.w);
-    }
+        if (solid) {
+            c.gv_s[n] = node_velocity_adj(S, s, ix, iy, D);
+            if (ZERO && tape_s) tape_s[n] = s;
+            (ZERO ? c.sum_s : c.ub_s)[n] = zero;
+        }
+        if (water) {
+            const float2 u = node_velocity_adj(S, w, ix, iy, D);
+            c.gv_w[n] = make_float4(u.x, u.y, w.x, w.w);
+            if (ZERO && tape_w) tape_w[n] = w;
+            (ZERO ? c.sum_w : c.ub_w)[n] = zero;
+        }
+    });
 }
 
 // The grid-update adjoint of the marked tiles' nodes, in place: the node
 // velocity adjoints that k_adj_g2p_bwd scattered become the adjoints of the
 // node sums (u = D (q / m + dt g): momentum q, mass m; the liquid volume's
 // passes through), once per node instead of once per particle reaching it.
-// One tile per CTA iteration, one node per thread.
-__global__ void __launch_bounds__(ADJ_TILE * ADJ_TILE) k_adj_grid_bwd(AdjCtx c, const uint32_t *tile_scene,
-                                                                      const uint32_t *list)
+__global__ void __launch_bounds__(ADJ_THREADS) k_adj_grid_bwd(AdjCtx c, const uint32_t *tile_scene, const uint8_t *mark,
+                                                              uint32_t n_tiles)
 {
-    const uint32_t count = list[0];
-    for (uint32_t i = blockIdx.x; i < count; i += gridDim.x) {
-        const uint32_t t = list[1 + i];
-        const AdjScene &S = c.scenes[tile_scene[t]];
-        const uint32_t local = t - S.tile_base;
-        const uint32_t hx = (local % S.tiles_x) * ADJ_TILE + threadIdx.x % ADJ_TILE;
-        const uint32_t hy = (local / S.tiles_x) * ADJ_TILE + threadIdx.x / ADJ_TILE;
-        if (hx >= S.node_w || hy >= S.cells_y + 3u) continue;
-        const uint32_t n = S.node_base + hy * S.node_w + hx;
-        const int ix = (int)hx - 1, iy = (int)hy - 1;
+    follow();
+    for_marked_nodes(c, tile_scene, mark, n_tiles, [&](const AdjScene &S, uint32_t n, int ix, int iy, bool solid, bool water) {
 #pragma unroll
         for (int channel = 0; channel < 2; ++channel) {
+            if (!(channel ? water : solid)) continue;
             float4 *ub = channel ? c.ub_w : c.ub_s;
             const float4 sum = channel ? c.sum_w[n] : c.sum_s[n];
             const float4 b = ub[n];  // velocity (x, y), liquid mass, liquid volume adjoints
@@ -555,14 +561,17 @@ __global__ void __launch_bounds__(ADJ_TILE * ADJ_TILE) k_adj_grid_bwd(AdjCtx c, 
             }
             ub[n] = make_float4(Qx_b, Qy_b, M_b, channel ? b.w : 0.f);
         }
-    }
+    });
 }
 
+// Loss sum |x - target|^2 per scene (one atomic per warp whose particles
+// share a scene) and its adjoint seeds.
 __global__ void __launch_bounds__(ADJ_THREADS) k_adj_loss(AdjCtx c)
 {
+    follow();
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     const bool valid = i < c.n;
-    const uint32_t scene = valid ? c.scene_of[i] : 0u;
+    const uint32_t scene = valid ? c.tag[i] >> 1 : 0u;
     double term = 0.0;
     if (valid) {
         const float2 x = c.in.x[i], t = c.target[i];
@@ -593,10 +602,12 @@ __global__ void __launch_bounds__(ADJ_THREADS, 3) k_adj_g2p_bwd(AdjCtx c)
     // recompute, read again by the adjoint's scatter
     __shared__ float2 s_u[9][ADJ_THREADS];
     __shared__ float2 s_mv[9][ADJ_THREADS];
+    follow();
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= c.n) return;
-    const AdjScene &S = c.scenes[c.scene_of[i]];
-    const bool liquid = c.liquid[i] != 0u;
+    const uint32_t tag = c.tag[i];
+    const AdjScene &S = c.scenes[tag >> 1];
+    const bool liquid = (tag & 1u) != 0u;
     const float2 x = c.in.x[i];
     const float4 F0 = c.in.F[i];
     AdjStencil st;
@@ -666,12 +677,12 @@ __global__ void __launch_bounds__(ADJ_THREADS, 3) k_adj_g2p_bwd(AdjCtx c)
         for (int ox = 0; ox < 3; ++ox) {
             const float w = st.wx[ox] * st.wy[oy];
             const float dpx = ((float)ox - st.fx) * S.dx;
-            const uint32_t n = adj_node(S, st.bx + ox, st.by + oy);
             const float2 u = s_u[oy * 3 + ox][threadIdx.x];
             const float2 mv = s_mv[oy * 3 + ox][threadIdx.x];  // liquid mass and volume
             // node velocity adjoint: w vpb + w Bb dp
             const float ubx = w * (vpb.x + Bb.x * dpx + Bb.y * dpy);
             const float uby = w * (vpb.y + Bb.z * dpx + Bb.w * dpy);
+            const uint32_t n = adj_node(S, st.bx + ox, st.by + oy);
             if (liquid)
                 atomicAdd(&c.ub_w[n], make_float4(ubx, uby, w * pm_b, w * pv_b));
             else
@@ -721,16 +732,17 @@ __device__ __forceinline__ void add_param_grads(double *grad, uint32_t scene, fl
 // reversed), then reverses its own P2G contribution and stress; adds the G2P
 // parts; writes the adjoints of the substep's inputs and the parameter
 // gradients.
-__global__ void __launch_bounds__(ADJ_THREADS, 3) k_adj_p2g_bwd(AdjCtx c)
+__global__ void __launch_bounds__(ADJ_THREADS, 4) k_adj_p2g_bwd(AdjCtx c)
 {
+    follow();
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     const bool valid = i < c.n;
-    const uint32_t scene = valid ? c.scene_of[i] : 0u;
+    const uint32_t tag = valid ? c.tag[i] : 0u, scene = tag >> 1;
     float3 pg = make_float3(0.f, 0.f, 0.f);
     bool ok = valid;
     if (valid) {
         const AdjScene &S = c.scenes[scene];
-        const bool liquid = c.liquid[i] != 0u;
+        const bool liquid = (tag & 1u) != 0u;
         const float2 x = c.in.x[i], v = c.in.v[i];
         const float4 C = c.in.C[i], F = c.in.F[i];
         const float vol = c.vol[i];
@@ -792,33 +804,39 @@ __global__ void __launch_bounds__(ADJ_THREADS, 3) k_adj_p2g_bwd(AdjCtx c)
 struct mpm_adjoint {
     int device = 0;
     cudaStream_t stream = nullptr;
+    RecordStage *stage = nullptr;  // pinned staging of the device
     uint32_t n = 0, n_scenes = 0, n_nodes = 0;
     std::vector<AdjScene> scenes;
     AdjScene *d_scenes = nullptr;
-    uint32_t *scene_of = nullptr, *liquid = nullptr, *status = nullptr;
+    uint32_t *tag = nullptr;
     float *vol = nullptr;
+    // the states of a run: init is state 0; checkpoint s (s > 0) state s * every;
+    // the others alternate in ping.  tape[j] and tape_s / tape_w[j]: state and
+    // sums of substep j of the segment tape_segment (-1: none yet).
     AdjState init{}, ping[2]{};
     std::vector<AdjState> checkpoints, tape;
-    float4 *sum_s = nullptr, *sum_w = nullptr;   // forward scratch
-    uint8_t *mark = nullptr;                     // per substep (0 .. steps) and clearing tile
+    std::vector<float4 *> tape_s, tape_w;
+    int tape_segment = -1;
+    float4 *sum_s = nullptr, *sum_w = nullptr;  // zero between substeps
+    uint8_t *mark = nullptr;                    // per substep (0 .. steps) and 16 x 16-node tile: solid, water
     size_t mark_count = 0;
-    uint32_t *lists = nullptr;                   // per substep: marked-tile count, then the tiles
-    uint32_t *tile_scene = nullptr;              // per clearing tile
-    uint32_t n_tiles = 0;
-    unsigned clear_ctas = 1;
-    std::vector<float4 *> tape_s, tape_w;       // per recomputed substep
+    uint32_t *tile_scene = nullptr;             // per tile
+    uint32_t n_tiles = 0, tile_ctas = 1;
     float2 *xb[2]{}, *vb[2]{}, *xg = nullptr;
     float4 *Cb[2]{}, *Fb[2]{}, *Fg = nullptr, *ub_w = nullptr, *ub_s = nullptr;
     float2 *gv_s = nullptr;  // node velocities of the substep at hand
     float4 *gv_w = nullptr;
-    double *param_grad = nullptr, *loss = nullptr;
+    // loss per scene, the status word (in 8 bytes), three parameter gradients per scene
+    double *results = nullptr;
     float2 *target = nullptr, *final_x = nullptr;
     uint32_t steps = 0, every = 0;
-    int final_buffer = 0;
     bool forward_done = false;
-    bool taped = false;  // the forward kept every substep's state and sums (one segment)
     cudaEvent_t ev[4]{};
     float forward_ms = 0.f, backward_ms = 0.f;
+
+    double *loss() const { return results; }
+    uint32_t *status() const { return reinterpret_cast<uint32_t *>(results + n_scenes); }
+    double *param_grad() const { return results + n_scenes + 1; }
 };
 
 namespace {
@@ -846,15 +864,6 @@ void free_state(AdjState &s)
     s = AdjState{};
 }
 
-cudaError_t copy_state(const AdjState &dst, const AdjState &src, size_t n, cudaStream_t st)
-{
-    cudaError_t e = cudaMemcpyAsync(dst.x, src.x, n * sizeof(float2), cudaMemcpyDeviceToDevice, st);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(dst.v, src.v, n * sizeof(float2), cudaMemcpyDeviceToDevice, st);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(dst.C, src.C, n * sizeof(float4), cudaMemcpyDeviceToDevice, st);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(dst.F, src.F, n * sizeof(float4), cudaMemcpyDeviceToDevice, st);
-    return e;
-}
-
 void free_engine(mpm_adjoint *a)
 {
     if (!a) return;
@@ -867,14 +876,15 @@ void free_engine(mpm_adjoint *a)
     for (auto &s : a->tape) free_state(s);
     for (float4 *p : a->tape_s) cudaFree(p);
     for (float4 *p : a->tape_w) cudaFree(p);
-    void *ptrs[] = {a->mark, a->lists, a->tile_scene, a->d_scenes, a->scene_of, a->liquid, a->status, a->vol, a->sum_s, a->sum_w, a->xb[0], a->xb[1],
-                    a->vb[0], a->vb[1], a->xg, a->ub_s, a->Cb[0], a->Cb[1], a->Fb[0], a->Fb[1], a->Fg, a->ub_w, a->gv_s, a->gv_w,
-                    a->param_grad, a->loss, a->target, a->final_x};
+    void *ptrs[] = {a->mark,  a->tile_scene, a->d_scenes, a->tag,   a->vol,   a->sum_s, a->sum_w,
+                    a->xb[0], a->xb[1],      a->vb[0],    a->vb[1], a->xg,    a->ub_s,  a->ub_w, a->Cb[0], a->Cb[1],
+                    a->Fb[0], a->Fb[1],      a->Fg,       a->gv_s,  a->gv_w,  a->results, a->target, a->final_x};
     for (void *p : ptrs)
         if (p) cudaFree(p);
     for (cudaEvent_t e : a->ev)
         if (e) cudaEventDestroy(e);
     if (a->stream) cudaStreamDestroy(a->stream);
+    if (a->stage) a->stage->release();
     delete a;
 }
 
@@ -898,11 +908,10 @@ AdjCtx make_adj_ctx(mpm_adjoint *a, const AdjState &in, const AdjState &out, flo
 {
     AdjCtx c{};
     c.scenes = a->d_scenes;
-    c.scene_of = a->scene_of;
-    c.liquid = a->liquid;
+    c.tag = a->tag;
     c.vol = a->vol;
     c.n = a->n;
-    c.status = a->status;
+    c.status = a->status();
     c.in = in;
     c.out = out;
     c.sum_s = sum_s;
@@ -918,62 +927,78 @@ AdjCtx make_adj_ctx(mpm_adjoint *a, const AdjState &in, const AdjState &out, flo
     c.xg = a->xg;
     c.Fg = a->Fg;
     c.ub_s = a->ub_s;
+    c.ub_w = a->ub_w;
     c.gv_s = a->gv_s;
     c.gv_w = a->gv_w;
-    c.ub_w = a->ub_w;
-    c.param_grad = a->param_grad;
+    c.param_grad = a->param_grad();
     c.target = a->target;
-    c.loss = a->loss;
+    c.loss = a->loss();
     return c;
 }
 
 unsigned blocks(uint32_t n) { return std::max(1u, (n + ADJ_THREADS - 1) / ADJ_THREADS); }
 
-// One forward substep from `in` to `out` with the sums in (ss, sw).
-// The clearing-tile marks of substep k (its input positions).
-uint8_t *marks_of(mpm_adjoint *a, uint32_t k) { return a->mark + (size_t)k * a->n_tiles; }
-
-// The marked-tile list of substep k.
-uint32_t *list_of(mpm_adjoint *a, uint32_t k) { return a->lists + (size_t)k * (a->n_tiles + 1u); }
-
-// Lists the marked tiles of substep k.
-void compact_marks(mpm_adjoint *a, uint32_t k)
+// Enqueues a kernel over the particles (one per thread) or over the tiles.
+template <class... Args>
+void over_particles(mpm_adjoint *a, void (*kernel)(Args...), Args... args)
 {
-    cudaMemsetAsync(list_of(a, k), 0, sizeof(uint32_t), a->stream);
-    k_adj_compact<<<blocks(a->n_tiles), COMPACT_THREADS, 0, a->stream>>>(marks_of(a, k), a->n_tiles, list_of(a, k));
+    launch_following(a->stream, kernel, dim3(blocks(a->n)), dim3(ADJ_THREADS), 0, args...);
 }
 
-// Zeroes the node arrays over the marked tiles of substep k (NULL arrays are skipped).
-void clear_marked(mpm_adjoint *a, uint32_t k, float4 *x, float4 *y, float2 *z)
+template <class... Args>
+void over_tiles(mpm_adjoint *a, void (*kernel)(Args...), Args... args)
 {
-    k_adj_clear<<<a->clear_ctas, ADJ_TILE * ADJ_TILE, 0, a->stream>>>(a->d_scenes, a->tile_scene, list_of(a, k), x, y,
-                                                                        z);
+    launch_following(a->stream, kernel, dim3(std::min(a->n_tiles, a->tile_ctas)), dim3(ADJ_THREADS), 0, args...);
 }
 
-// One forward substep k from `in` into `out`, its node sums in ss / sw: they
-// are zeroed over the substep's marked tiles first, and the new positions
-// mark substep k + 1's tiles (adding to the marks when a segment is
-// recomputed: float atomics may move a position by its last bits).
-cudaError_t forward_substep(mpm_adjoint *a, uint32_t k, const AdjState &in, const AdjState &out, float4 *ss, float4 *sw,
-                            bool run_g2p = true)
+// The tile marks of substep k (of its input positions).
+uint8_t *marks_of(mpm_adjoint *a, uint32_t k) { return a->mark + (size_t)k * a->n_tiles * 2u; }
+
+const uint32_t *tile_scenes(const mpm_adjoint *a) { return a->tile_scene; }
+const uint8_t *tile_marks(mpm_adjoint *a, uint32_t k) { return marks_of(a, k); }
+
+// The input state of substep k of the forward pass, whose last segment runs on
+// the tape (segment `last` from substep last * every).
+const AdjState &state_of(mpm_adjoint *a, uint32_t k, uint32_t last)
 {
-    clear_marked(a, k, ss, sw, nullptr);
-    AdjCtx c = make_adj_ctx(a, in, out, ss, sw, 0);
-    c.mark_out = marks_of(a, k + 1);
-    k_adj_p2g<<<blocks(a->n), ADJ_THREADS, 0, a->stream>>>(c);
-    if (run_g2p) {
-        k_adj_grid_fwd<<<a->clear_ctas, ADJ_TILE * ADJ_TILE, 0, a->stream>>>(c, a->tile_scene, list_of(a, k));
-        k_adj_g2p<<<blocks(a->n), ADJ_THREADS, 0, a->stream>>>(c);
-        compact_marks(a, k + 1);
+    if (k == 0u) return a->init;
+    if (k < a->steps && k % a->every == 0u) return a->checkpoints[k / a->every];
+    if (k < a->steps && k / a->every == last) return a->tape[k % a->every];
+    return a->ping[k & 1u];
+}
+
+// Substeps start .. start + len - 1 from state(start): the P2G of the first when
+// `p2g_first`, then per substep the grid update and G2P with the next P2G.
+// `tape` keeps the sums; the G2P of the last substep runs when `last_g2p`, with the
+// P2G after it when `last_p2g`.  Every P2G marks the tiles of its positions
+// (adding to the marks when a segment is recomputed: float atomics may move
+// a position by its last bits).
+template <class State>
+cudaError_t run_substeps(mpm_adjoint *a, uint32_t start, uint32_t len, const State &state, bool tape, bool p2g_first,
+                         bool last_g2p, bool last_p2g)
+{
+    if (p2g_first) {
+        AdjCtx c = make_adj_ctx(a, state(start), state(start), a->sum_s, a->sum_w, 0);
+        c.mark_out = marks_of(a, start);
+        over_particles(a, k_adj_p2g, c);
+    }
+    for (uint32_t j = 0; j < len; ++j) {
+        const uint32_t k = start + j;
+        AdjCtx c = make_adj_ctx(a, state(k), state(k + 1u), a->sum_s, a->sum_w, 0);
+        over_tiles(a, k_adj_grid_fwd<true>, c, tile_scenes(a), tile_marks(a, k), a->n_tiles,
+                   tape ? a->tape_s[j] : nullptr, tape ? a->tape_w[j] : nullptr);
+        if (j + 1u == len && !last_g2p) break;
+        c.mark_out = marks_of(a, k + 1u);
+        if (j + 1u < len || last_p2g)
+            over_particles(a, k_adj_g2p<true>, c);
+        else
+            over_particles(a, k_adj_g2p<false>, c);
     }
     return cudaGetLastError();
 }
 
-int check_status(mpm_adjoint *a, const char *what)
+int check_status(uint32_t st, const char *what)
 {
-    uint32_t st = 0;
-    ADJ_TRY(cudaMemcpyAsync(&st, a->status, sizeof st, cudaMemcpyDeviceToHost, a->stream));
-    ADJ_TRY(cudaStreamSynchronize(a->stream));
     if (st != 0u)
         return err(MPM_ERR_STATE, "%s stopped: %s%s%s", what, (st & ADJ_ERR_STENCIL) ? "a particle left the grid; " : "",
                    (st & ADJ_ERR_DETERMINANT) ? "a deformation gradient lost its positive determinant; " : "",
@@ -994,12 +1019,20 @@ int mpma_create(const mpm_config *configs, uint32_t scene_count, const uint32_t 
     *out = nullptr;
     if (scene_count < 1) return err(MPM_ERR_INVALID_ARGUMENT, "a batch needs at least one scene");
     std::vector<AdjScene> scenes(scene_count);
-    std::vector<uint32_t> scene_of, liquid;
+    std::vector<uint32_t> tag;
     std::vector<float> vol;
     std::vector<float2> x, v;
     std::vector<float4> C, F;
     uint64_t total = 0, nodes = 0;
-    std::vector<uint32_t> tile_scene;  // per clearing tile
+    std::vector<uint32_t> tile_scene;  // per tile
+    {
+        size_t all = 0;
+        for (uint32_t k = 0; k < scene_count; ++k) all += particle_counts[k];
+        for (auto *a : {&x, &v}) a->reserve(all);
+        for (auto *a : {&C, &F}) a->reserve(all);
+        vol.reserve(all);
+        tag.reserve(all);
+    }
     for (uint32_t k = 0; k < scene_count; ++k) {
         const mpm_config &cfg = configs[k];
         if (cfg.cells_x < 1 || cfg.cells_y < 1 || cfg.cells_x > 65536 || cfg.cells_y > 65536 || !(cfg.cell_size > 0.f))
@@ -1051,14 +1084,14 @@ int mpma_create(const mpm_config *configs, uint32_t scene_count, const uint32_t 
             C.push_back(make_float4(w[4], w[5], w[6], w[7]));
             F.push_back(make_float4(w[8], w[9], w[10], w[11]));
             vol.push_back(w[17]);
-            scene_of.push_back(k);
-            liquid.push_back(liq ? 1u : 0u);
+            tag.push_back((k << 1) | (liq ? 1u : 0u));
         }
         total += S.n;
         nodes += (uint64_t)(cfg.cells_x + 3) * (cfg.cells_y + 3);
         S.tile_base = (uint32_t)tile_scene.size();
         S.tiles_x = (cfg.cells_x + 3 + ADJ_TILE - 1) / ADJ_TILE;
         tile_scene.insert(tile_scene.end(), (size_t)S.tiles_x * ((cfg.cells_y + 3 + ADJ_TILE - 1) / ADJ_TILE), k);
+        // (this also keeps the tiles below 2^30)
         if (total > 0x7fffffffull || nodes > 0x7fffffffull)
             return err(MPM_ERR_INVALID_ARGUMENT, "the batch exceeds the GPU index range");
     }
@@ -1068,6 +1101,8 @@ int mpma_create(const mpm_config *configs, uint32_t scene_count, const uint32_t 
     ADJ_TRY(cudaSetDevice(device));
     mpm_adjoint *a = new mpm_adjoint();
     a->device = device;
+    a->stage = &RecordStage::of(device);
+    a->stage->retain();
     a->n = (uint32_t)total;
     a->n_scenes = scene_count;
     a->n_nodes = (uint32_t)nodes;
@@ -1087,9 +1122,7 @@ int mpma_create(const mpm_config *configs, uint32_t scene_count, const uint32_t 
         if (cudaEventCreate(&e) != cudaSuccess) return fail(err(MPM_ERR_CUDA, "cudaEventCreate failed"));
     const size_t n = a->n;
     ADJ_ALLOC(a->d_scenes, scene_count);
-    ADJ_ALLOC(a->scene_of, n);
-    ADJ_ALLOC(a->liquid, n);
-    ADJ_ALLOC(a->status, 1);
+    ADJ_ALLOC(a->tag, n);
     ADJ_ALLOC(a->vol, n);
     if (alloc_state(a->init, n) != cudaSuccess || alloc_state(a->ping[0], n) != cudaSuccess ||
         alloc_state(a->ping[1], n) != cudaSuccess)
@@ -1108,28 +1141,27 @@ int mpma_create(const mpm_config *configs, uint32_t scene_count, const uint32_t 
     ADJ_ALLOC(a->ub_w, nodes);
     ADJ_ALLOC(a->gv_s, nodes);
     ADJ_ALLOC(a->gv_w, nodes);
-    ADJ_ALLOC(a->param_grad, 3 * (size_t)scene_count);
-    ADJ_ALLOC(a->loss, scene_count);
+    ADJ_ALLOC(a->results, 4 * (size_t)scene_count + 1);
     ADJ_ALLOC(a->target, n);
     ADJ_ALLOC(a->final_x, n);
     a->n_tiles = (uint32_t)tile_scene.size();
     ADJ_ALLOC(a->tile_scene, tile_scene.size());
 #undef ADJ_ALLOC
-    {
-        int sms = 0;
-        if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess)
-            return fail(err(MPM_ERR_CUDA, "device query failed"));
-        a->clear_ctas = (unsigned)std::max<size_t>(1, std::min<size_t>(tile_scene.size(), (size_t)sms * 8));
-    }
+    int sms = 1;
+    if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess)
+        return fail(err(MPM_ERR_CUDA, "device query failed"));
+    a->tile_ctas = (uint32_t)sms * 8u;  // 2048 threads per SM
     bool ok = cudaMemcpy(a->d_scenes, scenes.data(), scene_count * sizeof(AdjScene), cudaMemcpyHostToDevice) == cudaSuccess;
-    ok = ok && cudaMemcpy(a->scene_of, scene_of.data(), n * sizeof(uint32_t), cudaMemcpyHostToDevice) == cudaSuccess;
-    ok = ok && cudaMemcpy(a->liquid, liquid.data(), n * sizeof(uint32_t), cudaMemcpyHostToDevice) == cudaSuccess;
+    ok = ok && cudaMemcpy(a->tag, tag.data(), n * sizeof(uint32_t), cudaMemcpyHostToDevice) == cudaSuccess;
     ok = ok && cudaMemcpy(a->vol, vol.data(), n * sizeof(float), cudaMemcpyHostToDevice) == cudaSuccess;
     ok = ok && cudaMemcpy(a->init.x, x.data(), n * sizeof(float2), cudaMemcpyHostToDevice) == cudaSuccess;
     ok = ok && cudaMemcpy(a->init.v, v.data(), n * sizeof(float2), cudaMemcpyHostToDevice) == cudaSuccess;
     ok = ok && cudaMemcpy(a->init.C, C.data(), n * sizeof(float4), cudaMemcpyHostToDevice) == cudaSuccess;
     ok = ok && cudaMemcpy(a->init.F, F.data(), n * sizeof(float4), cudaMemcpyHostToDevice) == cudaSuccess;
-    ok = ok && cudaMemset(a->status, 0, sizeof(uint32_t)) == cudaSuccess;
+    ok = ok && cudaMemset(a->results, 0, (4 * (size_t)scene_count + 1) * sizeof(double)) == cudaSuccess;
+    ok = ok && cudaMemset(a->sum_s, 0, nodes * sizeof(float4)) == cudaSuccess;
+    ok = ok && cudaMemset(a->sum_w, 0, nodes * sizeof(float4)) == cudaSuccess;
+    ok = ok && cudaDeviceSynchronize() == cudaSuccess;  // before work of the engine's own stream
     ok = ok && cudaMemcpy(a->tile_scene, tile_scene.data(), tile_scene.size() * sizeof(uint32_t),
                           cudaMemcpyHostToDevice) == cudaSuccess;
     if (!ok) return fail(err(MPM_ERR_CUDA, "upload failed"));
@@ -1172,7 +1204,7 @@ int mpma_set_velocities(mpm_adjoint *a, const float *velocities)
     host_clear_error();
     if (!a || !velocities) return err(MPM_ERR_INVALID_ARGUMENT, "engine and velocities must not be NULL");
     ADJ_TRY(cudaSetDevice(a->device));
-    ADJ_TRY(cudaMemcpy(a->init.v, velocities, (size_t)a->n * sizeof(float2), cudaMemcpyHostToDevice));
+    ADJ_TRY(a->stage->copy_in(a->stream, a->init.v, velocities, (size_t)a->n * sizeof(float2)));
     a->forward_done = false;
     return MPM_OK;
 }
@@ -1190,10 +1222,12 @@ int mpma_forward(mpm_adjoint *a, uint32_t substeps, const float *dts, uint32_t c
         a->scenes[k].dt = dts[k];
     }
     ADJ_TRY(cudaSetDevice(a->device));
-    ADJ_TRY(cudaMemcpy(a->d_scenes, a->scenes.data(), a->n_scenes * sizeof(AdjScene), cudaMemcpyHostToDevice));
-    ADJ_TRY(cudaMemcpy(a->target, targets, (size_t)a->n * sizeof(float2), cudaMemcpyHostToDevice));
+    ADJ_TRY(cudaMemcpyAsync(a->d_scenes, a->scenes.data(), a->n_scenes * sizeof(AdjScene), cudaMemcpyHostToDevice, a->stream));
+    ADJ_TRY(a->stage->copy_in(a->stream, a->target, targets, (size_t)a->n * sizeof(float2)));
     const uint32_t n_check = (substeps + checkpoint_every - 1) / checkpoint_every;
     if (a->checkpoints.size() != n_check || a->every != checkpoint_every) {
+        a->tape_segment = -1;
+        a->every = 0;
         for (auto &s : a->checkpoints) free_state(s);
         for (auto &s : a->tape) free_state(s);
         for (float4 *p : a->tape_s) cudaFree(p);
@@ -1202,68 +1236,49 @@ int mpma_forward(mpm_adjoint *a, uint32_t substeps, const float *dts, uint32_t c
         a->tape.assign(checkpoint_every, AdjState{});
         a->tape_s.assign(checkpoint_every, nullptr);
         a->tape_w.assign(checkpoint_every, nullptr);
-        for (auto &s : a->checkpoints)
-            if (alloc_state(s, a->n) != cudaSuccess) return err(MPM_ERR_CUDA, "checkpoint allocation failed");
+        // state 0 is the initial state, and substep 0 of a segment has its checkpoint
+        for (uint32_t k = 1; k < n_check; ++k)
+            if (alloc_state(a->checkpoints[k], a->n) != cudaSuccess) return err(MPM_ERR_CUDA, "checkpoint allocation failed");
         for (uint32_t j = 0; j < checkpoint_every; ++j) {
-            if (alloc_state(a->tape[j], a->n) != cudaSuccess || adj_alloc(&a->tape_s[j], a->n_nodes) != cudaSuccess ||
-                adj_alloc(&a->tape_w[j], a->n_nodes) != cudaSuccess)
+            if ((j > 0 && alloc_state(a->tape[j], a->n) != cudaSuccess) ||
+                adj_alloc(&a->tape_s[j], a->n_nodes) != cudaSuccess || adj_alloc(&a->tape_w[j], a->n_nodes) != cudaSuccess)
                 return err(MPM_ERR_CUDA, "recompute tape allocation failed");
         }
     }
     a->steps = substeps;
     a->every = checkpoint_every;
-    const size_t marks = ((size_t)substeps + 1) * a->n_tiles;
+    const size_t marks = ((size_t)substeps + 1) * a->n_tiles * 2;
     if (a->mark_count < marks) {
         cudaFree(a->mark);
         a->mark = nullptr;
         a->mark_count = 0;
-        cudaFree(a->lists);
-        a->lists = nullptr;
-        if (adj_alloc(&a->mark, marks) != cudaSuccess ||
-            adj_alloc(&a->lists, ((size_t)substeps + 1) * (a->n_tiles + 1u)) != cudaSuccess)
-            return err(MPM_ERR_CUDA, "tile mark allocation failed");
+        if (adj_alloc(&a->mark, marks) != cudaSuccess) return err(MPM_ERR_CUDA, "tile mark allocation failed");
         a->mark_count = marks;
     }
     ADJ_TRY(cudaMemsetAsync(a->mark, 0, marks, a->stream));
-    ADJ_TRY(cudaMemsetAsync(a->status, 0, sizeof(uint32_t), a->stream));
-    ADJ_TRY(cudaMemsetAsync(a->loss, 0, a->n_scenes * sizeof(double), a->stream));
+    ADJ_TRY(cudaMemsetAsync(a->results, 0, (a->n_scenes + 1) * sizeof(double), a->stream));
     ADJ_TRY(cudaEventRecord(a->ev[0], a->stream));
-    int cur = 0;
-    a->taped = n_check == 1;
-    if (a->taped) {
-        // one segment: the forward runs on the recompute tape itself (every
-        // substep's input state and node sums stay in HBM), so the backward
-        // pass recomputes nothing; the final state lands in ping[0]
-        ADJ_TRY(copy_state(a->tape[0], a->init, a->n, a->stream));
-        k_adj_mark<<<blocks(a->n), ADJ_THREADS, 0, a->stream>>>(
-            make_adj_ctx(a, a->tape[0], a->tape[0], nullptr, nullptr, 0), marks_of(a, 0));
-        compact_marks(a, 0);
-        for (uint32_t k = 0; k < substeps; ++k)
-            ADJ_TRY(forward_substep(a, k, a->tape[k], k + 1 < substeps ? a->tape[k + 1] : a->ping[0], a->tape_s[k],
-                                    a->tape_w[k]));
-    } else {
-        ADJ_TRY(copy_state(a->ping[0], a->init, a->n, a->stream));
-        k_adj_mark<<<blocks(a->n), ADJ_THREADS, 0, a->stream>>>(
-            make_adj_ctx(a, a->ping[0], a->ping[0], nullptr, nullptr, 0), marks_of(a, 0));
-        compact_marks(a, 0);
-        for (uint32_t k = 0; k < substeps; ++k) {
-            if (k % checkpoint_every == 0)
-                ADJ_TRY(copy_state(a->checkpoints[k / checkpoint_every], a->ping[cur], a->n, a->stream));
-            ADJ_TRY(forward_substep(a, k, a->ping[cur], a->ping[1 - cur], a->sum_s, a->sum_w));
-            cur = 1 - cur;
-        }
-    }
+    // the last segment (with checkpoint_every >= substeps the whole run) keeps
+    // its states and sums, so the backward pass does not recompute it
+    const uint32_t last = n_check - 1, last_start = last * checkpoint_every;
+    const auto state = [&](uint32_t k) -> const AdjState & { return state_of(a, k, last); };
+    if (last_start > 0) ADJ_TRY(run_substeps(a, 0, last_start, state, false, true, true, true));
+    ADJ_TRY(run_substeps(a, last_start, substeps - last_start, state, true, last_start == 0, true, false));
     ADJ_TRY(cudaEventRecord(a->ev[1], a->stream));
-    a->final_buffer = cur;
-    const AdjCtx c = make_adj_ctx(a, a->ping[cur], a->ping[cur], a->sum_s, a->sum_w, 0);
-    k_adj_loss<<<blocks(a->n), ADJ_THREADS, 0, a->stream>>>(c);
+    a->tape_segment = (int)last;
+    const AdjState &final_state = state(substeps);
+    over_particles(a, k_adj_loss, make_adj_ctx(a, final_state, final_state, a->sum_s, a->sum_w, 0));
     ADJ_TRY(cudaGetLastError());
-    ADJ_TRY(cudaMemcpyAsync(a->final_x, a->ping[cur].x, (size_t)a->n * sizeof(float2), cudaMemcpyDeviceToDevice,
-                            a->stream));
-    int rc = check_status(a, "the forward pass");
+    ADJ_TRY(cudaMemcpyAsync(a->final_x, final_state.x, (size_t)a->n * sizeof(float2), cudaMemcpyDeviceToDevice, a->stream));
+    std::vector<double> got(a->n_scenes + 1);
+    ADJ_TRY(cudaMemcpyAsync(got.data(), a->results, got.size() * sizeof(double), cudaMemcpyDeviceToHost, a->stream));
+    ADJ_TRY(cudaStreamSynchronize(a->stream));
+    uint32_t st;
+    std::memcpy(&st, &got[a->n_scenes], sizeof st);
+    const int rc = check_status(st, "the forward pass");
     if (rc != MPM_OK) return rc;
     ADJ_TRY(cudaEventElapsedTime(&a->forward_ms, a->ev[0], a->ev[1]));
-    if (loss) ADJ_TRY(cudaMemcpy(loss, a->loss, a->n_scenes * sizeof(double), cudaMemcpyDeviceToHost));
+    if (loss) std::memcpy(loss, got.data(), a->n_scenes * sizeof(double));
     a->forward_done = true;
     return MPM_OK;
 }
@@ -1274,36 +1289,47 @@ int mpma_backward(mpm_adjoint *a, float *grad_velocities, double *grad_parameter
     if (!a) return err(MPM_ERR_INVALID_ARGUMENT, "engine must not be NULL");
     if (!a->forward_done) return err(MPM_ERR_STATE, "backward needs a completed forward pass of the same inputs");
     ADJ_TRY(cudaSetDevice(a->device));
-    ADJ_TRY(cudaMemsetAsync(a->param_grad, 0, 3 * a->n_scenes * sizeof(double), a->stream));
+    ADJ_TRY(cudaMemsetAsync(a->param_grad(), 0, 3 * a->n_scenes * sizeof(double), a->stream));
     ADJ_TRY(cudaEventRecord(a->ev[2], a->stream));
     int adj = 0;  // the adjoint of the current substep's outputs sits in buffer `adj` (seeded by the loss)
     const uint32_t K = a->every;
     for (int seg = (int)a->checkpoints.size() - 1; seg >= 0; --seg) {
         const uint32_t start = (uint32_t)seg * K, len = std::min(K, a->steps - start);
-        if (!a->taped) ADJ_TRY(copy_state(a->tape[0], a->checkpoints[seg], a->n, a->stream));
-        for (uint32_t j = 0; j < len && !a->taped; ++j)
-            ADJ_TRY(forward_substep(a, start + j, a->tape[j], j + 1 < len ? a->tape[j + 1] : a->ping[0], a->tape_s[j],
-                                    a->tape_w[j], j + 1 < len));
+        // a substep's input state on the tape; the output of the last one is not kept
+        const auto state = [&](uint32_t k) -> const AdjState & {
+            if (k == start) return seg == 0 ? a->init : a->checkpoints[seg];
+            return k < start + len ? a->tape[k - start] : a->ping[0];
+        };
+        if (a->tape_segment != seg) {
+            a->tape_segment = -1;
+            ADJ_TRY(run_substeps(a, start, len, state, true, true, false, false));
+            a->tape_segment = seg;
+        }
         for (int j = (int)len - 1; j >= 0; --j) {
             const uint32_t k = start + (uint32_t)j;
-            clear_marked(a, k, a->ub_w, a->ub_s, nullptr);
-            const AdjCtx c = make_adj_ctx(a, a->tape[j], a->tape[j], a->tape_s[j], a->tape_w[j], adj);
-            k_adj_grid_fwd<<<a->clear_ctas, ADJ_TILE * ADJ_TILE, 0, a->stream>>>(c, a->tile_scene, list_of(a, k));
-            k_adj_g2p_bwd<<<blocks(a->n), ADJ_THREADS, 0, a->stream>>>(c);
-            k_adj_grid_bwd<<<a->clear_ctas, ADJ_TILE * ADJ_TILE, 0, a->stream>>>(c, a->tile_scene, list_of(a, k));
-            k_adj_p2g_bwd<<<blocks(a->n), ADJ_THREADS, 0, a->stream>>>(c);
+            const AdjCtx c = make_adj_ctx(a, state(k), state(k), a->tape_s[j], a->tape_w[j], adj);
+            over_tiles(a, k_adj_grid_fwd<false>, c, tile_scenes(a), tile_marks(a, k), a->n_tiles, (float4 *)nullptr,
+                       (float4 *)nullptr);
+            over_particles(a, k_adj_g2p_bwd, c);
+            over_tiles(a, k_adj_grid_bwd, c, tile_scenes(a), tile_marks(a, k), a->n_tiles);
+            over_particles(a, k_adj_p2g_bwd, c);
             adj = 1 - adj;
         }
         ADJ_TRY(cudaGetLastError());
     }
     ADJ_TRY(cudaEventRecord(a->ev[3], a->stream));
-    int rc = check_status(a, "the adjoint pass");
+    std::vector<double> got(3 * (size_t)a->n_scenes + 1);
+    ADJ_TRY(cudaMemcpyAsync(got.data(), a->results + a->n_scenes, got.size() * sizeof(double), cudaMemcpyDeviceToHost,
+                            a->stream));
+    ADJ_TRY(cudaStreamSynchronize(a->stream));
+    uint32_t st;
+    std::memcpy(&st, &got[0], sizeof st);
+    const int rc = check_status(st, "the adjoint pass");
     if (rc != MPM_OK) return rc;
     ADJ_TRY(cudaEventElapsedTime(&a->backward_ms, a->ev[2], a->ev[3]));
-    if (grad_velocities)
-        ADJ_TRY(cudaMemcpy(grad_velocities, a->vb[adj], (size_t)a->n * sizeof(float2), cudaMemcpyDeviceToHost));
-    if (grad_parameters)
-        ADJ_TRY(cudaMemcpy(grad_parameters, a->param_grad, 3 * a->n_scenes * sizeof(double), cudaMemcpyDeviceToHost));
+    const size_t bytes = (size_t)a->n * sizeof(float2);
+    if (grad_velocities) ADJ_TRY(a->stage->copy_out(a->stream, a->vb[adj], bytes, grad_velocities, bytes, nullptr));
+    if (grad_parameters) std::memcpy(grad_parameters, got.data() + 1, 3 * a->n_scenes * sizeof(double));
     return MPM_OK;
 }
 
@@ -1313,7 +1339,8 @@ int mpma_read_positions(mpm_adjoint *a, float *positions)
     if (!a || !positions) return err(MPM_ERR_INVALID_ARGUMENT, "engine and positions must not be NULL");
     if (!a->forward_done) return err(MPM_ERR_STATE, "no forward pass has completed");
     ADJ_TRY(cudaSetDevice(a->device));
-    ADJ_TRY(cudaMemcpy(positions, a->final_x, (size_t)a->n * sizeof(float2), cudaMemcpyDeviceToHost));
+    const size_t bytes = (size_t)a->n * sizeof(float2);
+    ADJ_TRY(a->stage->copy_out(a->stream, a->final_x, bytes, positions, bytes, nullptr));
     return MPM_OK;
 }
 

@@ -347,15 +347,6 @@ __device__ __forceinline__ void cp_async(void *dst, const void *src)
         asm volatile("cp.async.ca.shared.global [%0], [%1], %2;\n" ::"r"(d), "l"(src), "n"(N) : "memory");
 }
 
-// The start of a kernel of the substep chain: its CTAs may have been started
-// while the last CTAs of the kernel before it ended (a programmatic launch;
-// without one there is nothing to wait for); that kernel's results are complete
-// and visible from here on.  2-5 % of a substep at every size measured (1,600
-// particles 22.3 -> 21.8 us, 150,000 32.4 -> 31.0, 1,000,000 103.2 -> 103.0).
-// Letting the next kernel's CTAs start with this one's costs more than it gives:
-// they hold slots (1,000,000: 115.7 us).
-__device__ __forceinline__ void follow() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-
 __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;\n" ::: "memory"); }
 
 __device__ __forceinline__ uint32_t warp_sum(uint32_t v)

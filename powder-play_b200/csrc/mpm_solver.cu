@@ -20,6 +20,7 @@
 
 #include "../../include/mpm_b200.h"
 #include "mpm_kernels.cuh"
+#include "mpm_launch.cuh"
 #include "mpm_records.cuh"
 
 using namespace mpm;
@@ -230,17 +231,7 @@ bool uses_records(const mpm_solver *s)
 template <class... Args>
 void launch(mpm_solver *s, void (*kernel)(Args...), dim3 grid, dim3 block, size_t shared, Args... args)
 {
-    cudaLaunchConfig_t cfg{};
-    cfg.gridDim = grid;
-    cfg.blockDim = block;
-    cfg.dynamicSmemBytes = shared;
-    cfg.stream = s->stream;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    cudaLaunchKernelEx(&cfg, kernel, args...);
+    launch_following(s->stream, kernel, grid, block, shared, args...);
 }
 
 // Whether k_tile_bucket buckets the particles (else k_tile_alloc and
