@@ -193,7 +193,6 @@ def kernel_bytes(name: str, n: int, active: tuple) -> float:
         "k_grid_from_parts": channel_nodes * 32.0,
         "k_grid_update": channel_nodes * 32.0,
         "k_prepare_scatter": n * 56.0 + channel_nodes * 16.0,
-        "k_fixed_decode": channel_nodes * 16.0,
         # tile bucketing: reads x (8 B), writes key + rank (8 B); then reads
         # key + rank and writes the permutation (12 B)
         "k_tile_count": n * 16.0,

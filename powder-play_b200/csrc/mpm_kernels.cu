@@ -11,8 +11,7 @@
 // The cell sort (k_count, k_scan_*, k_scatter, k_stable_rank) backs the sort
 // probe and the allocation-free cell sort.
 // Substep, fixed-point atomic P2G (createExperimentalMpmMlsAtomicGpuSolver):
-//   k_substep_begin -> k_prepare_scatter -> k_fixed_decode -> k_grid_update
-//   -> k_g2p
+//   k_substep_begin -> k_prepare_scatter -> k_grid_update -> k_g2p
 // After a batch: k_end_batch (rollback, maximum particle speed).
 //
 // Every kernel returns early once the persistent status word is non-zero, as
@@ -1690,20 +1689,112 @@ __device__ __forceinline__ void add_sources(const Ctx &c, const NodeSources &ns,
 
 namespace {
 
-// addFixedPoint: shaders.ts:971-985.  The rounding is ties-to-even.
-__device__ __forceinline__ bool add_fixed(const Ctx &c, uint32_t index, float value)
+// Correctly rounded quotients by one divisor d, from its reciprocal r rounded
+// to nearest: q = a r is within two units in the last place of a / d, one
+// correction by the residual a - q d (a fused product) brings it within one, and a
+// second correction then rounds it to nearest for every d whose significand is not
+// all ones (P. Markstein, Computation of elementary functions on the IBM RISC
+// System/6000 processor, IBM J. Res. Dev. 34(1), 1990).  Five instructions and no
+// branch for each of a particle's 36 quotients.  A dividend so small that its residual
+// underflows has a quotient that rounds to the integer 0 (the scale is at most 2^30), one
+// so large that q overflows is out of the words' range.
+struct Quotient {
+    float d, r;
+    __device__ __forceinline__ explicit Quotient(float divisor)
+    {
+        d = divisor;
+        r = __frcp_rn(divisor);
+    }
+    __device__ __forceinline__ bool quick() const
+    {
+        const uint32_t bits = __float_as_uint(d);
+        const uint32_t exponent = (bits >> 23) & 0xffu;
+        return (bits & 0x7fffffu) != 0x7fffffu && exponent > 127u - 60u && exponent < 127u + 60u;
+    }
+    template <bool QUICK>
+    __device__ __forceinline__ float of(float a) const
+    {
+        if (!QUICK) return __fdiv_rn(a, d);
+        float q = __fmul_rn(a, r);
+        q = __fmaf_rn(__fmaf_rn(-q, d, a), r, q);
+        return __fmaf_rn(__fmaf_rn(-q, d, a), r, q);
+    }
+};
+
+// addFixedPoint (shaders.ts:971-985) in two halves.  The increment: the scaled
+// value rounded ties-to-even, false where it is not finite or above 2147483520 (a
+// float of that size is a whole number, so the bound holds before rounding too).
+__device__ __forceinline__ bool fixed_increment(float scaled, int32_t &inc)
 {
-    const float scaled = rintf(__fmul_rn(value, c.P->fixed_scale));
-    if (!finite_f(scaled) || fabsf(scaled) > 2147483520.0f) {
-        fail(c.status, ERROR_FIXED_POINT_RANGE);
-        return false;
+    inc = __float2int_rn(scaled);
+    return fabsf(scaled) <= 2147483520.0f;
+}
+
+// Its addition to a word that held prev: whether prev + inc leaves the range, as
+// the sign of the result.
+__device__ __forceinline__ int32_t fixed_overflow(int32_t prev, int32_t inc)
+{
+    const int32_t sum = (int32_t)((uint32_t)prev + (uint32_t)inc);
+    return (prev ^ sum) & (inc ^ sum);
+}
+
+// A particle's P2G for the fixed-point path.
+struct FixedParticle {
+    float4 A;
+    float mass, vliq;
+    float2 v;
+    Stencil s;
+    uint32_t orig;
+    int channel;  // first word of its channel (0 solid, 3 water, 7 oil)
+};
+
+// Calls add(ox, oy, word, increment) for the contributions of a particle, until
+// a node's raise a status.
+template <bool QUICK, class Add>
+__device__ __forceinline__ void fixed_contributions(const Ctx &c, const FixedParticle &p, const Add &add)
+{
+    const StepParams &P = *c.P;
+    const Quotient by_mass(P.particle_mass), by_volume(P.particle_volume);
+    const float scale = P.fixed_scale;
+    const bool liquid = p.channel != 0;
+#pragma unroll
+    for (int oy = 0; oy < 3; ++oy) {
+        const float wy = quad_weight(p.s.fy, oy);
+        const float dpy = __fmul_rn(__fsub_rn((float)oy, p.s.fy), P.dx);
+#pragma unroll
+        for (int ox = 0; ox < 3; ++ox) {
+            const float w = __fmul_rn(quad_weight(p.s.fx, ox), wy);
+            const float dpx = __fmul_rn(__fsub_rn((float)ox, p.s.fx), P.dx);
+            const float mx = __fadd_rn(__fadd_rn(__fmul_rn(p.mass, p.v.x), __fmul_rn(p.A.x, dpx)), __fmul_rn(p.A.y, dpy));
+            const float my = __fadd_rn(__fadd_rn(__fmul_rn(p.mass, p.v.y), __fmul_rn(p.A.z, dpx)), __fmul_rn(p.A.w, dpy));
+            int32_t inc[4];
+            bool fits = fixed_increment(__fmul_rn(by_mass.of<QUICK>(__fmul_rn(w, p.mass)), scale), inc[0]);
+            fits &= fixed_increment(__fmul_rn(by_mass.of<QUICK>(__fmul_rn(w, mx)), scale), inc[1]);
+            fits &= fixed_increment(__fmul_rn(by_mass.of<QUICK>(__fmul_rn(w, my)), scale), inc[2]);
+            fits &= !liquid | fixed_increment(__fmul_rn(by_volume.of<QUICK>(__fmul_rn(w, p.vliq)), scale), inc[3]);
+            if (!fits || !(w >= 0.0f)) {
+                // (a weight or momentum that is not finite gives no increment that fits)
+                if (!finite_f(w) || w < 0.0f || !finite_f(mx) || !finite_f(my))
+                    fail_at(c.status, p.orig, ERROR_P2G | ERROR_P2G_NONFINITE_PARTICLE);
+                else
+                    fail(c.status, ERROR_FIXED_POINT_RANGE);
+                return;
+            }
+            add(ox, oy, 0, inc[0]);
+            add(ox, oy, 1, inc[1]);
+            add(ox, oy, 2, inc[2]);
+            if (liquid) add(ox, oy, 3, inc[3]);
+        }
     }
-    const int32_t inc = (int32_t)scaled;
-    const int32_t prev = atomicAdd(&c.fixed[index], inc);
-    if ((inc > 0 && prev > 2147483647 - inc) || (inc < 0 && prev < (-2147483647 - 1) - inc)) {
-        fail(c.status, ERROR_FIXED_POINT_RANGE);
-    }
-    return true;
+}
+
+template <class Add>
+__device__ __forceinline__ void fixed_contributions(const Ctx &c, const FixedParticle &p, const Add &add)
+{
+    if (Quotient(c.P->particle_mass).quick() && Quotient(c.P->particle_volume).quick())
+        fixed_contributions<true>(c, p, add);
+    else
+        fixed_contributions<false>(c, p, add);
 }
 
 }  // namespace
@@ -1711,112 +1802,197 @@ __device__ __forceinline__ bool add_fixed(const Ctx &c, uint32_t index, float va
 // prepareAndScatterParticles: shaders.ts:987-1043.  Integer sums are
 // order-independent, so this path is bit-reproducible and is checked
 // bit-exactly against a CPU emulation of the same integers.
-__global__ void k_prepare_scatter(Ctx c)
+//
+// 36 global atomics per liquid particle would bind it to L2's atomic rate
+// (240,000 particles: 72 us a launch).  The particles of a CTA are neighbours
+// in the uploaded order and stay so for a long time: a CTA whose stencils lie in
+// a box of at most SCATTER_WORDS words sums its integers in shared memory
+// and adds each non-zero word once: 19 us, bound by the issue of the 36
+// quotients and sums of a particle in 1.6 rounds of CTAs (256 threads a CTA: 20.5
+// us, 128: 21; 40 registers for a third CTA per SM: no gain).  A CTA whose box is larger, or one of whose partial sums leaves the
+// range (the sum over all particles may not), adds every contribution itself.
+__global__ void __launch_bounds__(SCATTER_THREADS, 2) k_prepare_scatter(Ctx c)
 {
     follow();
     const StepParams &P = *c.P;
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= P.n_particles) return;
-    if (*(volatile uint32_t *)c.status != 0u) return;
-    float4 A;
-    float mass, vliq;
-    uint32_t model;
-    if (!prepare_particle(c, i, A, mass, vliq, model)) return;
-    if (c.affine_out) c.affine_out[i] = A;
-    if (*(volatile uint32_t *)c.status != 0u) return;
-    Stencil s;
-    if (!make_stencil(P, c.in.pos[i], s) || !stencil_fits(P, s.bx, s.by)) {
-        fail(c.status, ERROR_STENCIL);
-        return;
+    __shared__ __align__(16) int32_t s_word[SCATTER_WORDS];
+    __shared__ int s_box[4];  // least and greatest halo node of the stencils' base nodes: x, y
+    __shared__ uint32_t s_channels;
+    __shared__ int s_stop, s_over;
+    if (threadIdx.x == 0) {
+        s_stop = *(volatile uint32_t *)c.status != 0u ? 1 : 0;  // one read for the CTA
+        s_box[0] = s_box[2] = 0x7fffffff;
+        s_box[1] = s_box[3] = -1;
+        s_channels = 0u;
+        s_over = 0;
     }
-    const uint32_t stamp = c.counters[COUNTER_STAMP];
-    const uint32_t hx0 = (uint32_t)(s.bx + 1), hy0 = (uint32_t)(s.by + 1);
-    c.tile_stamp[tile_of_node(P, hx0, hy0)] = stamp;
-    c.tile_stamp[tile_of_node(P, hx0 + 2, hy0)] = stamp;
-    c.tile_stamp[tile_of_node(P, hx0, hy0 + 2)] = stamp;
-    c.tile_stamp[tile_of_node(P, hx0 + 2, hy0 + 2)] = stamp;
-    const float2 v = c.in.vel[i];
-    const bool liquid = model == MODEL_WATER || model == MODEL_OIL;
-    const uint32_t channel = model == MODEL_WATER ? 3u : (model == MODEL_OIL ? 7u : 0u);
-    const float pm = P.particle_mass, pv = P.particle_volume;
-    for (int oy = 0; oy < 3; ++oy) {
-        for (int ox = 0; ox < 3; ++ox) {
-            const float w = __fmul_rn(quad_weight(s.fx, ox), quad_weight(s.fy, oy));
-            const float dpx = __fmul_rn(__fsub_rn((float)ox, s.fx), P.dx);
-            const float dpy = __fmul_rn(__fsub_rn((float)oy, s.fy), P.dx);
-            const float mx = __fadd_rn(__fadd_rn(__fmul_rn(mass, v.x), __fmul_rn(A.x, dpx)), __fmul_rn(A.y, dpy));
-            const float my = __fadd_rn(__fadd_rn(__fmul_rn(mass, v.y), __fmul_rn(A.z, dpx)), __fmul_rn(A.w, dpy));
-            if (!finite_f(w) || w < 0.0f || !finite_f(mx) || !finite_f(my)) {
-                fail_at(c.status, c.in.orig[i], ERROR_P2G | ERROR_P2G_NONFINITE_PARTICLE);
-                return;
-            }
-            const uint32_t field = node_index(P, s.bx + ox, s.by + oy) * FIXED_WORDS + channel;
-            if (!add_fixed(c, field, __fdiv_rn(__fmul_rn(w, mass), pm))) return;
-            if (!add_fixed(c, field + 1, __fdiv_rn(__fmul_rn(w, mx), pm))) return;
-            if (!add_fixed(c, field + 2, __fdiv_rn(__fmul_rn(w, my), pm))) return;
-            if (liquid && !add_fixed(c, field + 3, __fdiv_rn(__fmul_rn(w, vliq), pv))) return;
+    __syncthreads();
+    if (s_stop) return;
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    FixedParticle p;
+    bool valid = i < P.n_particles;
+    uint32_t model = 0u;
+    float2 pos = make_float2(0.f, 0.f);
+    if (valid) {
+        pos = c.in.pos[i];
+        p.v = c.in.vel[i];
+        p.orig = c.in.orig[i];
+    }
+    if (valid && prepare_particle(c, i, p.A, p.mass, p.vliq, model)) {
+        if (c.affine_out) c.affine_out[i] = p.A;
+        if (!make_stencil(P, pos, p.s) || !stencil_fits(P, p.s.bx, p.s.by)) {
+            fail(c.status, ERROR_STENCIL);
+            valid = false;
+        }
+    } else {
+        valid = false;
+    }
+    const int hx0 = valid ? p.s.bx + 1 : 0, hy0 = valid ? p.s.by + 1 : 0;
+    if (valid) {
+        const uint32_t stamp = c.counters[COUNTER_STAMP];
+        const uint32_t tx = (uint32_t)hx0, ty = (uint32_t)hy0;
+        c.tile_stamp[tile_of_node(P, tx, ty)] = stamp;
+        c.tile_stamp[tile_of_node(P, tx + 2, ty)] = stamp;
+        c.tile_stamp[tile_of_node(P, tx, ty + 2)] = stamp;
+        c.tile_stamp[tile_of_node(P, tx + 2, ty + 2)] = stamp;
+        p.channel = model == MODEL_WATER ? 3 : (model == MODEL_OIL ? 7 : 0);
+    }
+    {
+        const int x_lo = __reduce_min_sync(0xffffffffu, valid ? hx0 : 0x7fffffff), x_hi = __reduce_max_sync(0xffffffffu, valid ? hx0 : -1);
+        const int y_lo = __reduce_min_sync(0xffffffffu, valid ? hy0 : 0x7fffffff), y_hi = __reduce_max_sync(0xffffffffu, valid ? hy0 : -1);
+        const uint32_t bit = valid ? (p.channel == 0 ? 1u : (p.channel == 3 ? 2u : 4u)) : 0u;
+        const uint32_t bits = __reduce_or_sync(0xffffffffu, bit);
+        if ((threadIdx.x & 31u) == 0u && bits != 0u) {
+            atomicMin(&s_box[0], x_lo);
+            atomicMax(&s_box[1], x_hi);
+            atomicMin(&s_box[2], y_lo);
+            atomicMax(&s_box[3], y_hi);
+            atomicOr(&s_channels, bits);
         }
     }
-}
-
-// gatherAtomicGrid: shaders.ts:1045-1070.  Decodes and clears the integer
-// words of every node of a touched tile.  Decoding ignores the status word so
-// the accumulators are always clean for the next substep.
-__global__ void __launch_bounds__(TILE_NODES) k_fixed_decode(Ctx c)
-{
-    follow();
-    const StepParams &P = *c.P;
-    const int tx = blockIdx.x, ty = blockIdx.y;
-    if (c.tile_stamp[ty * P.tiles_x + tx] != c.counters[COUNTER_STAMP]) return;
-    const int hx = tx * TILE_X + (threadIdx.x % TILE_X), hy = ty * TILE_Y + (threadIdx.x / TILE_X);
-    if (hx >= (int)P.node_w || hy >= (int)P.node_h) return;
-    const uint32_t n = (uint32_t)hy * P.node_w + (uint32_t)hx;
-    int32_t *w = c.fixed + (size_t)n * FIXED_WORDS;
-    float v[FIXED_WORDS];
-    const float inv = 1.0f / P.fixed_scale;
+    __syncthreads();
+    const uint32_t channels = s_channels;
+    if (channels == 0u) return;
+    // the box's words: four for each node (a solid one's last is idle), row by row,
+    // channel by channel of those present
+    const int x0 = s_box[0], y0 = s_box[2];
+    const uint32_t box_w = (uint32_t)(s_box[1] - x0) + 3u, box_h = (uint32_t)(s_box[3] - y0) + 3u;
+    const uint64_t plane64 = (uint64_t)box_w * box_h * 4u;
+    bool direct = plane64 * __popc(channels) > SCATTER_WORDS;
+    if (!direct) {
+        const uint32_t plane = (uint32_t)plane64, words = plane * __popc(channels);
+        for (uint32_t k = threadIdx.x; k < words / 4u; k += SCATTER_THREADS)
+            reinterpret_cast<int4 *>(s_word)[k] = make_int4(0, 0, 0, 0);
+        __syncthreads();
+        if (valid) {
+            const uint32_t before = p.channel == 0 ? 0u : (p.channel == 3 ? channels & 1u : __popc(channels & 3u));
+            int32_t *const word = s_word + before * plane + ((uint32_t)(hy0 - y0) * box_w + (uint32_t)(hx0 - x0)) * 4u;
+            int32_t over = 0;
+            fixed_contributions(c, p, [&](int ox, int oy, int k, int32_t inc) {
+                over |= fixed_overflow(atomicAdd(word + ((uint32_t)oy * box_w + (uint32_t)ox) * 4u + (uint32_t)k, inc), inc);
+            });
+            if (over < 0) s_over = 1;
+        }
+        __syncthreads();
+        direct = s_over != 0;
+        // (node / box_w by a product: exact, as both are below 2^16)
+        const uint32_t inverse = 0xffffffffu / box_w + 1u;
+        uint32_t first = 0u;
+        for (uint32_t channel = 0u; channel < 3u && !direct; ++channel) {
+            if (((channels >> channel) & 1u) == 0u) continue;
+            const uint32_t field = channel == 0u ? 0u : 4u * channel - 1u;
+            // (four sums of a thread in flight: each waits for L2's answer)
+            for (uint32_t k0 = threadIdx.x; k0 < plane; k0 += 4u * SCATTER_THREADS) {
+                int32_t inc[4], prev[4];
 #pragma unroll
-    for (int k = 0; k < FIXED_WORDS; ++k) {
-        v[k] = (float)w[k] * inv;
-        w[k] = 0;
+                for (uint32_t u = 0u; u < 4u; ++u) {
+                    const uint32_t k = k0 + u * SCATTER_THREADS;
+                    inc[u] = k < plane ? s_word[first + k] : 0;
+                    const uint32_t node = k / 4u, row = __umulhi(node, inverse), column = node - row * box_w;
+                    const uint32_t n = ((uint32_t)y0 + row) * P.node_w + (uint32_t)x0 + column;
+                    prev[u] = inc[u] != 0 ? atomicAdd(&c.fixed[(size_t)n * FIXED_WORDS + field + k % 4u], inc[u]) : 0;
+                }
+#pragma unroll
+                for (int u = 0; u < 4; ++u)
+                    if (fixed_overflow(prev[u], inc[u]) < 0) fail(c.status, ERROR_FIXED_POINT_RANGE);
+            }
+            first += plane;
+        }
     }
-    if (*(volatile uint32_t *)c.status != 0u) return;
-    const float pm = P.particle_mass, pv = P.particle_volume;
-    c.p2g_solid[n] = make_float4(v[0] * pm, v[1] * pm, v[2] * pm, 0.f);
-    c.p2g_water[n] = make_float4(v[3] * pm, v[4] * pm, v[5] * pm, v[6] * pv);
-    c.p2g_oil[n] = make_float4(v[7] * pm, v[8] * pm, v[9] * pm, v[10] * pv);
+    if (direct && valid) {
+        fixed_contributions(c, p, [&](int ox, int oy, int k, int32_t inc) {
+            const size_t n = node_index(P, p.s.bx + ox, p.s.by + oy);
+            if (fixed_overflow(atomicAdd(&c.fixed[n * FIXED_WORDS + (uint32_t)(p.channel + k)], inc), inc) < 0)
+                fail(c.status, ERROR_FIXED_POINT_RANGE);
+        });
+    }
 }
 
 namespace {
 
-// volumeAtNode: shaders.ts:1779-1790, reading zero for tiles that no particle
-// touched this substep (their storage is stale, not cleared).
-__device__ __forceinline__ float2 phase_volume(const Ctx &c, int hx, int hy, uint32_t stamp)
+// Decoded water and oil volumes of a halo node (volumeAtNode,
+// shaders.ts:1779-1790): zero outside the halo; a node no particle reached holds zero words.
+__device__ __forceinline__ float2 phase_volume(const Ctx &c, int hx, int hy, float inv)
 {
     const StepParams &P = *c.P;
     if (hx < 0 || hy < 0 || hx >= (int)P.node_w || hy >= (int)P.node_h) return make_float2(0.f, 0.f);
-    if (c.tile_stamp[tile_of_node(P, (uint32_t)hx, (uint32_t)hy)] != stamp) return make_float2(0.f, 0.f);
-    const uint32_t n = (uint32_t)hy * P.node_w + (uint32_t)hx;
-    return make_float2(c.p2g_water[n].w, c.p2g_oil[n].w);
+    const int32_t *w = c.fixed + ((size_t)hy * P.node_w + (size_t)hx) * FIXED_WORDS;
+    const float pv = P.particle_volume;
+    return make_float2((float)w[6] * inv * pv, (float)w[10] * inv * pv);
+}
+
+// Calls work(tile) for each tile of the last substep's stamp that is dealt to
+// CTA `cta` of `ctas`, all THREADS threads together; the CTA reads the stamps of THREADS of
+// its tiles at once.
+template <int THREADS, class Work>
+__device__ __forceinline__ void for_stamped_tiles(const Ctx &c, uint32_t cta, uint32_t ctas, const Work &work)
+{
+    __shared__ uint32_t s_tile[THREADS], s_count;
+    const uint32_t stamp = c.counters[COUNTER_STAMP], n_tiles = c.P->tiles_x * c.P->tiles_y;
+    for (uint64_t first = cta; first < n_tiles; first += (uint64_t)ctas * THREADS) {
+        __syncthreads();
+        if (threadIdx.x == 0) s_count = 0u;
+        __syncthreads();
+        const uint64_t t = first + (uint64_t)threadIdx.x * ctas;
+        if (t < n_tiles && c.tile_stamp[t] == stamp) s_tile[atomicAdd(&s_count, 1u)] = (uint32_t)t;
+        __syncthreads();
+        const uint32_t count = s_count;
+        for (uint32_t k = 0; k < count; ++k) work(s_tile[k]);
+    }
 }
 
 }  // namespace
 
-// updateGrid of the fixed-point path: the same node update over the decoded
-// sums of touched tiles.
+// gatherAtomicGrid (shaders.ts:1045-1070) and updateGrid of the fixed-point
+// path: each node of a touched tile decodes its integer words and its
+// neighbours' volumes and writes its velocities.  The words are cleared by
+// k_g2p.  The tiles are dealt to the CTAs, which read the stamps of theirs
+// together.
 __global__ void __launch_bounds__(TILE_NODES) k_grid_update(Ctx c)
 {
     follow();
     const StepParams &P = *c.P;
-    const int tx = blockIdx.x, ty = blockIdx.y;
-    const uint32_t stamp = c.counters[COUNTER_STAMP];
-    if (c.tile_stamp[ty * P.tiles_x + tx] != stamp) return;
-    if (*(volatile uint32_t *)c.status != 0u) return;
-    const int hx = tx * TILE_X + (threadIdx.x % TILE_X), hy = ty * TILE_Y + (threadIdx.x / TILE_X);
-    if (hx >= (int)P.node_w || hy >= (int)P.node_h) return;
-    const uint32_t n = (uint32_t)hy * P.node_w + (uint32_t)hx;
-    update_node(c, n, hx - 1, hy - 1, c.p2g_solid[n], c.p2g_water[n], c.p2g_oil[n],
-                phase_volume(c, hx + 1, hy, stamp), phase_volume(c, hx - 1, hy, stamp),
-                phase_volume(c, hx, hy + 1, stamp), phase_volume(c, hx, hy - 1, stamp));
+    __shared__ int s_stop;
+    if (threadIdx.x == 0) s_stop = *(volatile uint32_t *)c.status != 0u ? 1 : 0;
+    __syncthreads();
+    if (s_stop) return;
+    const float inv = 1.0f / P.fixed_scale, pm = P.particle_mass, pv = P.particle_volume;
+    for_stamped_tiles<TILE_NODES>(c, blockIdx.x, gridDim.x, [&](uint32_t tile) {
+        const int hx = (int)(tile % P.tiles_x) * TILE_X + (int)(threadIdx.x % TILE_X);
+        const int hy = (int)(tile / P.tiles_x) * TILE_Y + (int)(threadIdx.x / TILE_X);
+        if (hx >= (int)P.node_w || hy >= (int)P.node_h) return;
+        const uint32_t n = (uint32_t)hy * P.node_w + (uint32_t)hx;
+        const int32_t *w = c.fixed + (size_t)n * FIXED_WORDS;
+        float v[FIXED_WORDS];
+#pragma unroll
+        for (int u = 0; u < FIXED_WORDS; ++u) v[u] = (float)w[u] * inv;
+        const float4 S = make_float4(v[0] * pm, v[1] * pm, v[2] * pm, 0.f);
+        const float4 W = make_float4(v[3] * pm, v[4] * pm, v[5] * pm, v[6] * pv);
+        const float4 O = make_float4(v[7] * pm, v[8] * pm, v[9] * pm, v[10] * pv);
+        c.node_channels[n] = (uint8_t)((S.x > 0.f ? 1 : 0) | (W.x > 0.f ? 2 : 0) | (O.x > 0.f ? 4 : 0));
+        update_node(c, n, hx - 1, hy - 1, S, W, O, phase_volume(c, hx + 1, hy, inv), phase_volume(c, hx - 1, hy, inv),
+                    phase_volume(c, hx, hy + 1, inv), phase_volume(c, hx, hy - 1, inv));
+    });
 }
 
 // ------------------------------------------------------------------ G2P --
@@ -2243,42 +2419,41 @@ __device__ __forceinline__ bool g2p_particle(const Ctx &c, const ParticleIn &in,
 
 // g2p: shaders.ts:2114-2421 (APIC velocity and affine C, liquid
 // density-contrast acceleration, adaptive fused F update with retries,
-// per-model projection, wall confinement, fused CFL validation).  Thread d
-// takes the particle at sorted position d (slot perm[d]) and writes slot d,
-// so the output is sorted by cell; in the gather path it also counts the
-// particle's new base cell for the next substep's sort.
-__global__ void k_g2p(Ctx c)
+// per-model projection, wall confinement, fused CFL validation) of the
+// fixed-point path: thread d takes the particle in slot d and writes slot d.
+// Four CTAs per SM (64 registers): 240,000 particles take 12.5 us, with three
+// 14.3, with five 13.4, the clearing included.
+__global__ void __launch_bounds__(PARTICLE_THREADS, 4) k_g2p(Ctx c)
 {
     follow();
     const StepParams &P = *c.P;
-    const uint32_t d = blockIdx.x * blockDim.x + threadIdx.x;
-    const bool in_range = d < P.n_particles;
-    const uint32_t s = in_range ? (c.perm ? c.perm[d] : d) : 0u;
-    bool counted = false;
-    uint32_t key = 0;
-    if (in_range) {
-        if (*(volatile uint32_t *)c.status != 0u) {
-            // the substep is rolled back: the batch ends on its input
-        } else {
-            const ParticleIn in = load_particle(c, s);
-            Stencil st, next;
-            if (!make_stencil(P, in.pos, st) || !stencil_fits(P, st.bx, st.by)) {
-                fail(c.status, ERROR_STENCIL);
-            } else {
-                const GlobalGrid grid{c.g_solid, c.g_water, c.g_oil, node_index(P, st.bx, st.by), P.node_w};
-                bool count_it;
-                if (g2p_particle<true, false, false>(c, in, d, st, grid, next, count_it) && count_it) {
-                    key = particle_tile(P, next.bx, next.by);
-                    counted = true;
-                }
+    const uint32_t particle_ctas = (P.n_particles + PARTICLE_THREADS - 1) / PARTICLE_THREADS;
+    if (blockIdx.x >= particle_ctas) {
+        // the touched tiles' words are cleared for the next substep (whatever the
+        // status: the accumulators are always clean), after the grid update read them
+        for_stamped_tiles<PARTICLE_THREADS>(c, blockIdx.x - particle_ctas, gridDim.x - particle_ctas, [&](uint32_t tile) {
+            const uint32_t x0 = tile % P.tiles_x * TILE_X, y0 = tile / P.tiles_x * TILE_Y;
+            const uint32_t row = min((uint32_t)TILE_X, P.node_w - x0) * FIXED_WORDS;
+            for (uint32_t k = threadIdx.x; k < TILE_X * FIXED_WORDS * TILE_Y; k += PARTICLE_THREADS) {
+                const uint32_t y = y0 + k / (TILE_X * FIXED_WORDS), word = k % (TILE_X * FIXED_WORDS);
+                if (y < P.node_h && word < row) c.fixed[((size_t)y * P.node_w + x0) * FIXED_WORDS + word] = 0;
             }
+        });
+        return;
+    }
+    const uint32_t d = blockIdx.x * PARTICLE_THREADS + threadIdx.x;
+    // (once the status is raised the substep is rolled back: the batch ends on its input)
+    if (d < P.n_particles && *(volatile uint32_t *)c.status == 0u) {
+        const ParticleIn in = load_particle(c, d);
+        Stencil st, next;
+        if (!make_stencil(P, in.pos, st) || !stencil_fits(P, st.bx, st.by)) {
+            fail(c.status, ERROR_STENCIL);
+        } else {
+            const GlobalGrid grid{c.g_solid, c.g_water, c.g_oil, node_index(P, st.bx, st.by), P.node_w};
+            bool count_it;
+            g2p_particle<true, false, false>(c, in, d, st, grid, next, count_it);
         }
     }
-    if (!c.count_next) return;
-    const unsigned active = __ballot_sync(0xffffffffu, counted);
-    if (!counted) return;
-    c.ranks[d] = warp_count(c.tile_count, key, active);
-    c.keys[d] = key;
 }
 
 namespace {
@@ -2806,7 +2981,7 @@ __global__ void k_end_batch(Ctx c0, uint32_t total, uint32_t measure_speed)
 
 // Counts the nodes of the last fixed-point substep whose solid / water / oil
 // mass is positive (the N_ch of the algorithmic-byte model), over stamped
-// tiles.  The default path counts them inside k_grid_from_acc instead.
+// tiles, as k_grid_update left them.
 __global__ void __launch_bounds__(TILE_NODES) k_count_active_nodes(Ctx c, uint32_t *counts)
 {
     const StepParams &P = *c.P;
@@ -2814,13 +2989,8 @@ __global__ void __launch_bounds__(TILE_NODES) k_count_active_nodes(Ctx c, uint32
     // the stamp of the last substep is still current
     if (c.tile_stamp[ty * P.tiles_x + tx] != c.counters[COUNTER_STAMP]) return;
     const int hx = tx * TILE_X + (threadIdx.x % TILE_X), hy = ty * TILE_Y + (threadIdx.x / TILE_X);
-    uint32_t s = 0, w = 0, o = 0;
-    if (hx < (int)P.node_w && hy < (int)P.node_h) {
-        const uint32_t n = (uint32_t)hy * P.node_w + (uint32_t)hx;
-        s = c.p2g_solid[n].x > 0.f;
-        w = c.p2g_water[n].x > 0.f;
-        o = c.p2g_oil[n].x > 0.f;
-    }
+    const uint32_t mask = hx < (int)P.node_w && hy < (int)P.node_h ? c.node_channels[(uint32_t)hy * P.node_w + (uint32_t)hx] : 0u;
+    uint32_t s = mask & 1u, w = (mask >> 1) & 1u, o = mask >> 2;
     s = __reduce_add_sync(0xffffffffu, s);
     w = __reduce_add_sync(0xffffffffu, w);
     o = __reduce_add_sync(0xffffffffu, o);

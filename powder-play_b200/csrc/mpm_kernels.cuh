@@ -19,7 +19,7 @@
 //     mask) pair, and the list of tiles holding particles; updated velocities solid
 //     float2, water float4 (vx,vy,mass_l,vol_l), oil float4 -- exactly what
 //     G2P reads per channel.  The reference-exact fixed-point path adds 11
-//     i32 words per node, its decoded sums 3 x float4, and one stamp u32 per
+//     i32 words per node, a byte of channels, and one stamp u32 per
 //     tile (tiles touched this substep).
 #pragma once
 
@@ -97,9 +97,7 @@ struct Ctx {
     float2 *rec_mom;     // m v
     uint32_t *rec_cell;  // local cell in its tile | channel << 8 | REC_FAILED
     // grid
-    float4 *p2g_solid;
-    float4 *p2g_water;
-    float4 *p2g_oil;
+    uint8_t *node_channels;  // fixed-point path: channels with positive mass per node of the last substep
     float2 *g_solid;
     float4 *g_water;
     float4 *g_oil;
@@ -163,6 +161,10 @@ constexpr int END_BATCH_THREADS = 256;      // k_end_batch: threads per CTA and
 constexpr int END_BATCH_ITEMS = 4;          // particles per thread and pass
 static_assert(VOL_X * VOL_Y <= G2P_THREADS && RING_NODES <= G2P_THREADS, "one node per thread");
 
+constexpr int PARTICLE_THREADS = 256;     // kernels of a thread per particle
+constexpr int SCATTER_THREADS = 512;      // k_prepare_scatter: particles per CTA and
+constexpr uint32_t SCATTER_WORDS = 8192;  // words it can sum in shared memory
+
 // device counters beyond the three of mpm_device.cuh
 constexpr int COUNTER_SUBSTEP = 8;       // the substep of this batch under way (failed and skipped included)
 constexpr int COUNTER_FRESH = 9;         // 1 from the start of a batch until its first substep starts
@@ -212,7 +214,6 @@ size_t substep_shared_bytes(int cap);
 template <bool SCENES, bool BODIES, bool LIQ, bool REC>
 __global__ void k_g2p_tile(Ctx c);
 __global__ void k_prepare_scatter(Ctx c);
-__global__ void k_fixed_decode(Ctx c);
 __global__ void k_grid_update(Ctx c);
 __global__ void k_g2p(Ctx c);
 __global__ void k_substep_begin(Ctx c);

@@ -120,7 +120,7 @@ struct mpm_solver {
 
     uint32_t *keys = nullptr, *ranks = nullptr, *tmp = nullptr, *perm = nullptr;
     uint32_t *cell_count = nullptr, *cell_start = nullptr, *block_sums = nullptr;
-    float4 *p2g_solid = nullptr, *p2g_water = nullptr, *p2g_oil = nullptr;
+    uint8_t *node_channels = nullptr;
     float2 *g_solid = nullptr;
     float4 *g_water = nullptr, *g_oil = nullptr;
     int32_t *fixed = nullptr;
@@ -267,9 +267,7 @@ Ctx make_ctx(mpm_solver *s, int parity)
     c.block_sums = s->block_sums;
     c.cell_pad = s->cell_pad;
     c.count_next = s->gather() ? 1u : 0u;
-    c.p2g_solid = s->p2g_solid;
-    c.p2g_water = s->p2g_water;
-    c.p2g_oil = s->p2g_oil;
+    c.node_channels = s->node_channels;
     c.g_solid = s->g_solid;
     c.g_water = s->g_water;
     c.g_oil = s->g_oil;
@@ -313,16 +311,15 @@ Ctx make_ctx(mpm_solver *s, int parity)
 
 inline unsigned blocks_for(uint32_t n, unsigned threads) { return std::max(1u, (n + threads - 1) / threads); }
 
-constexpr unsigned PARTICLE_THREADS = 256;
 
 // Kernel slots of the profiled substep (mpm_profile_substeps).
 enum KernelSlot {
     K_TILE_COUNT, K_TILE_ALLOC, K_TILE_SCATTER, K_P2G_GATHER, K_G2P_TILE, K_PREPARE_SCATTER,
-    K_FIXED_DECODE, K_GRID_UPDATE, K_G2P, K_SUBSTEP_BEGIN, K_END_BATCH, K_SUBSTEP, K_TILE_BUCKET, K_SLOTS
+    K_GRID_UPDATE, K_G2P, K_SUBSTEP_BEGIN, K_END_BATCH, K_SUBSTEP, K_TILE_BUCKET, K_SLOTS
 };
 const char *const KERNEL_NAMES[K_SLOTS] = {
     "k_tile_count", "k_tile_alloc", "k_tile_scatter", "k_p2g_gather", "k_g2p_tile", "k_prepare_scatter",
-    "k_fixed_decode", "k_grid_update", "k_g2p", "k_substep_begin", "k_end_batch", "k_substep", "k_tile_bucket"};
+    "k_grid_update", "k_g2p", "k_substep_begin", "k_end_batch", "k_substep", "k_tile_bucket"};
 
 // When set, an event is recorded after every kernel launch so that the
 // kernels of a substep can be timed one by one.  The profiled substeps are
@@ -532,7 +529,6 @@ void launch_g2p(mpm_solver *s, const Ctx &c, bool liq)
 void enqueue_substep(mpm_solver *s, int parity)
 {
     const Ctx c = make_ctx(s, parity);
-    const unsigned pb = blocks_for(s->n, PARTICLE_THREADS);
     const dim3 tiles(s->tiles_x, s->tiles_y);
     if (runs_fused(s)) {
         const cudaError_t e = launch_substep(s, c);
@@ -565,14 +561,12 @@ void enqueue_substep(mpm_solver *s, int parity)
     } else {
         launch(s, k_substep_begin, dim3(blocks_for(s->n_scenes, PARTICLE_THREADS)), dim3(PARTICLE_THREADS), 0, c);
         mark(K_SUBSTEP_BEGIN);
-        launch(s, k_prepare_scatter, dim3(pb), dim3(PARTICLE_THREADS), 0, c);
+        launch(s, k_prepare_scatter, dim3(blocks_for(s->n, SCATTER_THREADS)), dim3(SCATTER_THREADS), 0, c);
         mark(K_PREPARE_SCATTER);
-        launch(s, k_fixed_decode, tiles, dim3(TILE_NODES), 0, c);
-        mark(K_FIXED_DECODE);
         if (s->n_bodies) launch(s, k_triangle_field, tiles, dim3(TILE_NODES), 0, c);
-        launch(s, k_grid_update, tiles, dim3(TILE_NODES), 0, c);
+        launch(s, k_grid_update, dim3(std::min(s->tiles_x * s->tiles_y, s->sms * 16u)), dim3(TILE_NODES), 0, c);
         mark(K_GRID_UPDATE);
-        launch(s, k_g2p, dim3(pb), dim3(PARTICLE_THREADS), 0, c);
+        launch(s, k_g2p, dim3(blocks_for(s->n, PARTICLE_THREADS) + std::min(s->tiles_x * s->tiles_y, s->sms)), dim3(PARTICLE_THREADS), 0, c);
         mark(K_G2P);
     }
     enqueue_bodies(s, c);
@@ -860,8 +854,7 @@ void free_solver(mpm_solver *s)
     if (s->stream) cudaStreamSynchronize(s->stream);
     drop_graphs(s);
     void *ptrs[] = {s->d_params, s->dyn, s->work, s->tile_scene, s->scene_p_base, s->bonded, s->obj, s->d_mats, s->keys, s->ranks,
-                    s->tmp, s->perm, s->cell_count, s->cell_start, s->block_sums, s->p2g_solid, s->p2g_water,
-                    s->p2g_oil, s->g_solid, s->g_water, s->g_oil, s->fixed, s->tile_stamp, s->d_active,
+                    s->tmp, s->perm, s->cell_count, s->cell_start, s->block_sums, s->node_channels, s->g_solid, s->g_water, s->g_oil, s->fixed, s->tile_stamp, s->d_active,
                     s->tile_count, s->tile_range, s->scene_chunk, s->active_tiles, s->part, s->tile_info,
                     s->field, s->body_starts,
                     s->slot_of[0], s->slot_of[1], s->track_flag, s->tracked, s->pair_cache, s->contact_count,
@@ -1100,6 +1093,10 @@ int create_impl(const mpm_config *configs, uint32_t n_scenes, const uint32_t *co
                 cudaSuccess)
             return fail(set_error(MPM_ERR_CUDA, "scene table upload failed"));
     }
+    int sms = 0;
+    if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, s->device) != cudaSuccess)
+        return fail(set_error(MPM_ERR_CUDA, "device query failed"));
+    s->sms = (unsigned)sms;
     if (c.p2g_mode == MPM_P2G_GATHER) {
         ALLOC(s->active_tiles, n_tiles * (1 + G2P_MAX_PARTS));
         ALLOC(s->part, n_tiles * ACC_WORDS * RING_NODES);
@@ -1111,23 +1108,19 @@ int create_impl(const mpm_config *configs, uint32_t n_scenes, const uint32_t *co
         if (cudaMemsetAsync(s->tile_info, 0xff, n_tiles * sizeof(uint2), s->stream) != cudaSuccess ||
             cudaMemsetAsync(s->tile_count, 0, n_tiles * sizeof(uint32_t), s->stream) != cudaSuccess)
             return fail(set_error(MPM_ERR_CUDA, "cudaMemset failed"));
-        int sms = 0, per_sm_p2g = 0, per_sm_g2p = 0, per_sm_substep = 0;
+        int per_sm_p2g = 0, per_sm_g2p = 0, per_sm_substep = 0;
         if (configure_variant_kernels() != cudaSuccess ||
-            cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, s->device) != cudaSuccess ||
             variant_occupancy(s->stage_cap, &per_sm_p2g, &per_sm_substep) != cudaSuccess ||
             cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm_g2p, k_g2p_tile<false, false, false, false>, G2P_THREADS, 0) !=
                 cudaSuccess)
             return fail(set_error(MPM_ERR_CUDA, "occupancy query failed"));
-        s->sms = (unsigned)sms;
         s->p2g_ctas = (unsigned)std::max<size_t>(1, std::min<size_t>(n_tiles, (size_t)sms * std::max(1, per_sm_p2g)));
         s->g2p_ctas = (unsigned)std::max<size_t>(1, std::min<size_t>(n_tiles * G2P_MAX_PARTS, (size_t)sms * std::max(1, per_sm_g2p)));
         s->substep_max_ctas = (unsigned)std::max(1, sms * per_sm_substep);
         s->substep_ctas = s->substep_max_ctas;
     }
     if (c.p2g_mode == MPM_P2G_FIXED_POINT) {
-        ALLOC(s->p2g_solid, s->node_count);
-        ALLOC(s->p2g_water, s->node_count);
-        ALLOC(s->p2g_oil, s->node_count);
+        ALLOC(s->node_channels, s->node_count);
         ALLOC(s->fixed, (size_t)s->node_count * FIXED_WORDS);
         if (cudaMemsetAsync(s->fixed, 0, (size_t)s->node_count * FIXED_WORDS * sizeof(int32_t), s->stream) != cudaSuccess)
             return fail(set_error(MPM_ERR_CUDA, "cudaMemset failed"));
@@ -2331,7 +2324,7 @@ int mpm_probe_fixed_point(mpm_solver *s, float dt, int32_t *words_out, float *af
     CUDA_TRY(dalloc(&aff, s->n));
     Ctx c = make_ctx(s, s->cur);
     c.affine_out = aff;
-    k_prepare_scatter<<<blocks_for(s->n, PARTICLE_THREADS), PARTICLE_THREADS, 0, s->stream>>>(c);
+    k_prepare_scatter<<<blocks_for(s->n, SCATTER_THREADS), SCATTER_THREADS, 0, s->stream>>>(c);
     cudaError_t e = cudaGetLastError();
     const size_t words = (size_t)s->node_count * FIXED_WORDS;
     if (e == cudaSuccess && words_out)
