@@ -162,7 +162,7 @@ constexpr int END_BATCH_ITEMS = 4;          // particles per thread and pass
 static_assert(VOL_X * VOL_Y <= G2P_THREADS && RING_NODES <= G2P_THREADS, "one node per thread");
 
 constexpr int PARTICLE_THREADS = 256;     // kernels of a thread per particle
-constexpr int SCATTER_THREADS = 512;      // k_prepare_scatter: particles per CTA and
+constexpr int SCATTER_THREADS = 512;      // k_prepare_scatter, k_surface_gather: particles per CTA and
 constexpr uint32_t SCATTER_WORDS = 8192;  // words it can sum in shared memory
 
 // device counters beyond the three of mpm_device.cuh
@@ -245,7 +245,7 @@ struct SurfaceGeometry {
     uint32_t cells_x, cells_y, node_w;
 };
 __global__ void k_surface_gather(Ctx c, SurfaceGeometry g, unsigned long long *acc);
-__global__ void k_surface_decode(const unsigned long long *acc, float2 *field, uint32_t nodes);
+__global__ void k_surface_decode(unsigned long long *acc, float2 *field, uint32_t nodes, const uint32_t *flags);
 // interaction
 __global__ void k_outlet_compact(Ctx c, float4 bounds, ParticleBuffers removed, uint32_t *counters);
 __global__ void k_pick(Ctx c, float px, float py, float r2, unsigned long long *best);

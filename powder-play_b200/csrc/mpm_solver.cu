@@ -2137,26 +2137,35 @@ int mpm_gather_surface_occupancy(mpm_solver *s, float *field_out, uint32_t *surf
     CUDA_TRY(cudaSetDevice(s->device));
     const uint32_t nodes = s->node_count;
     if (!s->surface_acc) {
-        CUDA_TRY(dalloc(&s->surface_acc, 2 * (size_t)nodes));
-        CUDA_TRY(dalloc(&s->surface_field, nodes));
+        unsigned long long *acc = nullptr;
+        float2 *field = nullptr;
+        cudaError_t e = dalloc(&acc, 2 * (size_t)nodes);
+        if (e == cudaSuccess) e = dalloc(&field, (size_t)nodes + 1);  // the last holds the flags
+        if (e == cudaSuccess) e = cudaMemsetAsync(acc, 0, 2 * (size_t)nodes * sizeof(unsigned long long), s->stream);
+        if (e != cudaSuccess) {
+            cudaFree(acc);
+            cudaFree(field);
+            CUDA_TRY(e);
+        }
+        s->surface_acc = acc;
+        s->surface_field = field;
     }
-    CUDA_TRY(cudaMemsetAsync(s->surface_acc, 0, 2 * (size_t)nodes * sizeof(unsigned long long), s->stream));
     const SurfaceGeometry g{s->cfg.cell_size, s->cfg.cells_x, s->cfg.cells_y, s->node_w};
     if (s->n > 0) {
         const Ctx c = make_ctx(s, s->cur);
-        k_surface_gather<<<blocks_for(s->n, PARTICLE_THREADS), PARTICLE_THREADS, 0, s->stream>>>(c, g, s->surface_acc);
-        CUDA_TRY(cudaGetLastError());
+        CUDA_TRY(launch_following(s->stream, k_surface_gather, dim3(blocks_for(s->n, SCATTER_THREADS)), dim3(SCATTER_THREADS), 0,
+                                  c, g, s->surface_acc));
     }
-    k_surface_decode<<<blocks_for(nodes, PARTICLE_THREADS), PARTICLE_THREADS, 0, s->stream>>>(s->surface_acc,
-                                                                                           s->surface_field, nodes);
-    CUDA_TRY(cudaGetLastError());
+    CUDA_TRY(launch_following(s->stream, k_surface_decode, dim3(blocks_for(nodes, PARTICLE_THREADS)), dim3(PARTICLE_THREADS), 0,
+                              s->surface_acc, s->surface_field, nodes, (const uint32_t *)(s->d_status + 7)));
+    uint32_t flags = 0u;
+    const size_t bytes = (size_t)nodes * sizeof(float2);
     if (field_out)
-        CUDA_TRY(cudaMemcpyAsync(field_out, s->surface_field, (size_t)nodes * sizeof(float2), cudaMemcpyDeviceToHost,
-                                 s->stream));
-    if (surface_flags_out)
-        CUDA_TRY(cudaMemcpyAsync(surface_flags_out, s->d_status + 7, sizeof(uint32_t), cudaMemcpyDeviceToHost,
-                                 s->stream));
+        CUDA_TRY(s->stage->copy_out(s->stream, s->surface_field, bytes + sizeof(uint32_t), field_out, bytes, &flags));
+    else
+        CUDA_TRY(cudaMemcpyAsync(&flags, s->surface_field + nodes, sizeof(uint32_t), cudaMemcpyDeviceToHost, s->stream));
     CUDA_TRY(cudaStreamSynchronize(s->stream));
+    if (surface_flags_out) *surface_flags_out = flags;
     return MPM_OK;
 }
 
