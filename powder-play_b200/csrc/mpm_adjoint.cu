@@ -90,6 +90,7 @@ struct AdjCtx {
     float4 *Fg;            // the G2P part of the input F adjoint
     float4 *ub_s;          // per node: solid velocity adjoint (x, y), then (Qx, Qy, M) adjoints, 0
     float4 *ub_w;          // per node: water velocity, liquid mass, liquid volume adjoints
+    float4 *ub_s_prev, *ub_w_prev;  // those of the substep before, while the pass turns to it
     double *param_grad;    // per scene: tait, lambda_s, mu_s
     const float2 *target;  // per particle
     double *loss;          // per scene
@@ -288,13 +289,8 @@ struct G2pFwd {
     float2 xn;       // new position before confinement
 };
 
-// With `keep_u` / `keep_mv` (shared memory, [stencil node][ADJ_THREADS]) it
-// also keeps each stencil node's velocity and, for a liquid, its liquid mass
-// and volume, for this thread's adjoint.
-template <bool KEEP = false>
 __device__ __forceinline__ bool g2p_forward(const AdjCtx &c, const AdjScene &S, bool liquid, const AdjStencil &st,
-                                            float2 x, float4 F0, G2pFwd &g, float2 (*keep_u)[ADJ_THREADS] = nullptr,
-                                            float2 (*keep_mv)[ADJ_THREADS] = nullptr)
+                                            float2 x, float4 F0, G2pFwd &g)
 {
     g.vp = make_float2(0.f, 0.f);
     g.B = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -316,10 +312,6 @@ __device__ __forceinline__ bool g2p_forward(const AdjCtx &c, const AdjScene &S, 
                 sum.w = gw.w;
             } else {
                 u = c.gv_s[n];
-            }
-            if constexpr (KEEP) {
-                keep_u[oy * 3 + ox][threadIdx.x] = u;
-                keep_mv[oy * 3 + ox][threadIdx.x] = make_float2(sum.x, sum.w);
             }
             g.vp.x += w * u.x;
             g.vp.y += w * u.y;
@@ -470,14 +462,15 @@ __global__ void __launch_bounds__(ADJ_THREADS, 4) k_adj_g2p(AdjCtx c)
 // lies in a marked tile, and the rest of the grid keeps stale values that no
 // stencil reads.  The tiles are dealt to the CTAs one by one (marked ones lie
 // together), a CTA reads the marks of its tiles together and then visits the
-// marked ones: visit(scene, node, x, y, solid, water).  No list of the marked
+// marked ones: visit(scene, node, x, y, marks), marks 1 for solid and 2 for water,
+// four times as much by the marks of the substep before.  No list of the marked
 // tiles is built and no node cleared ahead of a substep: the grid update leaves the
 // sums at zero.  64 scenes of 16,384 particles, 200 substeps forward and backward:
-// 8 + 7 launches per substep -> 2 + 6, 73.9 -> 55.6 ms; one scene of 1,024, 40
-// substeps: 2.08 -> 0.93 ms.
+// 8 launches per substep forward and 7 backward -> 2 and 2 (and 2 to recompute a
+// segment), 73.9 -> 48.9 ms; one scene of 1,024, 40 substeps: 2.08 -> 0.76 ms.
 template <class Visit>
 __device__ __forceinline__ void for_marked_nodes(const AdjCtx &c, const uint32_t *tile_scene, const uint8_t *mark,
-                                                 uint32_t n_tiles, const Visit &visit)
+                                                 const uint8_t *mark_prev, uint32_t n_tiles, const Visit &visit)
 {
     __shared__ uint32_t s_tile[ADJ_THREADS], s_count;
     for (uint32_t first = blockIdx.x; first < n_tiles; first += gridDim.x * ADJ_THREADS) {
@@ -486,82 +479,114 @@ __device__ __forceinline__ void for_marked_nodes(const AdjCtx &c, const uint32_t
         __syncthreads();
         const uint64_t t = first + (uint64_t)threadIdx.x * gridDim.x;
         if (t < n_tiles) {
-            const uint32_t both = reinterpret_cast<const uint16_t *>(mark)[t];  // 1: solid, 0x100: water
-            if (both != 0u) s_tile[atomicAdd(&s_count, 1u)] = (uint32_t)t << 2 | (both & 1u) | (both >> 7 & 2u);
+            // 1: solid, 0x100: water, four times as much for the substep before
+            uint32_t both = reinterpret_cast<const uint16_t *>(mark)[t];
+            if (mark_prev) both |= (uint32_t)reinterpret_cast<const uint16_t *>(mark_prev)[t] << 2;
+            if (both != 0u) s_tile[atomicAdd(&s_count, 1u)] = (uint32_t)t << 4 | (both & 5u) | (both >> 7 & 10u);
         }
         __syncthreads();
         const uint32_t count = s_count;
         for (uint32_t k = 0; k < count; ++k) {
-            const uint32_t entry = s_tile[k], tile = entry >> 2;
+            const uint32_t entry = s_tile[k], tile = entry >> 4;
             const AdjScene &S = c.scenes[tile_scene[tile]];
             const uint32_t local = tile - S.tile_base;
             const uint32_t hx = (local % S.tiles_x) * ADJ_TILE + threadIdx.x % ADJ_TILE;
             const uint32_t hy = (local / S.tiles_x) * ADJ_TILE + threadIdx.x / ADJ_TILE;
             if (hx < S.node_w && hy < S.cells_y + 3u)
-                visit(S, S.node_base + hy * S.node_w + hx, (int)hx - 1, (int)hy - 1, (entry & 1u) != 0u, (entry & 2u) != 0u);
+                visit(S, S.node_base + hy * S.node_w + hx, (int)hx - 1, (int)hy - 1, entry & 15u);
         }
     }
 }
 
 // The grid update (finishGridVelocity with the wall factors,
-// node_velocity_adj): each node's velocity from its sums, for the G2P kernels;
-// the water record also carries the node's liquid mass and volume.  ZERO: the
-// sums are scratch; they are kept in tape_s / tape_w (unless NULL) and zeroed
-// for the next P2G.  Else the sums are a kept substep's, and the node adjoints
-// are zeroed for the G2P adjoint.
+// node_velocity_adj) of one node: its velocity from its sums, for the G2P
+// kernels; the water record also carries the node's liquid mass and volume.
+__device__ __forceinline__ void grid_velocity(const AdjCtx &c, const AdjScene &S, uint32_t n, int ix, int iy, bool solid,
+                                              bool water, float4 s, float4 w)
+{
+    float2 D;
+    if (solid) c.gv_s[n] = node_velocity_adj(S, s, ix, iy, D);
+    if (water) {
+        const float2 u = node_velocity_adj(S, w, ix, iy, D);
+        c.gv_w[n] = make_float4(u.x, u.y, w.x, w.w);
+    }
+}
+
+// The grid update of the marked tiles' nodes.  ZERO: the sums are scratch; they
+// are kept in tape_s / tape_w (unless NULL) and zeroed for the next P2G.  Else the
+// sums are a kept substep's, and the node adjoints are zeroed for the G2P
+// adjoint.
 template <bool ZERO>
 __global__ void __launch_bounds__(ADJ_THREADS) k_adj_grid_fwd(AdjCtx c, const uint32_t *tile_scene, const uint8_t *mark,
                                                               uint32_t n_tiles, float4 *tape_s, float4 *tape_w)
 {
     follow();
     const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
-    for_marked_nodes(c, tile_scene, mark, n_tiles, [&](const AdjScene &S, uint32_t n, int ix, int iy, bool solid, bool water) {
+    for_marked_nodes(c, tile_scene, mark, nullptr, n_tiles, [&](const AdjScene &S, uint32_t n, int ix, int iy, uint32_t marks) {
+        const bool solid = (marks & 1u) != 0u, water = (marks & 2u) != 0u;
         float4 s, w;
         if (solid) s = c.sum_s[n];
         if (water) w = c.sum_w[n];
-        float2 D;
+        grid_velocity(c, S, n, ix, iy, solid, water, s, w);
         if (solid) {
-            c.gv_s[n] = node_velocity_adj(S, s, ix, iy, D);
             if (ZERO && tape_s) tape_s[n] = s;
             (ZERO ? c.sum_s : c.ub_s)[n] = zero;
         }
         if (water) {
-            const float2 u = node_velocity_adj(S, w, ix, iy, D);
-            c.gv_w[n] = make_float4(u.x, u.y, w.x, w.w);
             if (ZERO && tape_w) tape_w[n] = w;
             (ZERO ? c.sum_w : c.ub_w)[n] = zero;
         }
     });
 }
 
-// The grid-update adjoint of the marked tiles' nodes, in place: the node
-// velocity adjoints that k_adj_g2p_bwd scattered become the adjoints of the
-// node sums (u = D (q / m + dt g): momentum q, mass m; the liquid volume's
-// passes through), once per node instead of once per particle reaching it.
+// The grid-update adjoint of one node and channel: the node velocity
+// adjoints that the G2P adjoint scattered, b = (velocity x, y, liquid mass, liquid volume), to
+// the adjoints of the node sums (u = D (q / m + dt g): momentum q, mass m; the
+// liquid volume's passes through), once per node instead of once per particle
+// reaching it.
+__device__ __forceinline__ float4 grid_adjoint(const AdjScene &S, int ix, int iy, bool water, float4 sum, float4 b)
+{
+    float M_b = water ? b.z : 0.f, Qx_b = 0.f, Qy_b = 0.f;
+    if (sum.x > 0.0f) {
+        float2 D;
+        node_velocity_adj(S, sum, ix, iy, D);
+        const float inv = 1.0f / sum.x;
+        const float udx = D.x * b.x, udy = D.y * b.y;
+        Qx_b = udx * inv;
+        Qy_b = udy * inv;
+        M_b -= (udx * sum.y + udy * sum.z) * inv * inv;
+    }
+    return make_float4(Qx_b, Qy_b, M_b, water ? b.w : 0.f);
+}
+
+// The grid-update adjoint of the marked tiles' nodes, in place.  TURN: and the
+// grid update of the substep before, whose sums and marks are given, with its node
+// adjoints zeroed, as k_adj_grid_fwd<false> does it: one launch and one pass over
+// the tiles fewer per substep.
+template <bool TURN>
 __global__ void __launch_bounds__(ADJ_THREADS) k_adj_grid_bwd(AdjCtx c, const uint32_t *tile_scene, const uint8_t *mark,
-                                                              uint32_t n_tiles)
+                                                              const uint8_t *mark_prev, uint32_t n_tiles,
+                                                              const float4 *prev_s, const float4 *prev_w)
 {
     follow();
-    for_marked_nodes(c, tile_scene, mark, n_tiles, [&](const AdjScene &S, uint32_t n, int ix, int iy, bool solid, bool water) {
-#pragma unroll
-        for (int channel = 0; channel < 2; ++channel) {
-            if (!(channel ? water : solid)) continue;
-            float4 *ub = channel ? c.ub_w : c.ub_s;
-            const float4 sum = channel ? c.sum_w[n] : c.sum_s[n];
-            const float4 b = ub[n];  // velocity (x, y), liquid mass, liquid volume adjoints
-            float M_b = channel ? b.z : 0.f, Qx_b = 0.f, Qy_b = 0.f;
-            if (sum.x > 0.0f) {
-                float2 D;
-                node_velocity_adj(S, sum, ix, iy, D);
-                const float inv = 1.0f / sum.x;
-                const float udx = D.x * b.x, udy = D.y * b.y;
-                Qx_b = udx * inv;
-                Qy_b = udy * inv;
-                M_b -= (udx * sum.y + udy * sum.z) * inv * inv;
-            }
-            ub[n] = make_float4(Qx_b, Qy_b, M_b, channel ? b.w : 0.f);
-        }
-    });
+    const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+    for_marked_nodes(c, tile_scene, mark, TURN ? mark_prev : nullptr, n_tiles,
+                     [&](const AdjScene &S, uint32_t n, int ix, int iy, uint32_t marks) {
+                         const bool solid = (marks & 1u) != 0u, water = (marks & 2u) != 0u;
+                         const bool solid_prev = TURN && (marks & 4u) != 0u, water_prev = TURN && (marks & 8u) != 0u;
+                         float4 s, w, us, uw, ps, pw;
+                         if (solid) s = c.sum_s[n], us = c.ub_s[n];
+                         if (water) w = c.sum_w[n], uw = c.ub_w[n];
+                         if (solid_prev) ps = prev_s[n];
+                         if (water_prev) pw = prev_w[n];
+                         if (solid) c.ub_s[n] = grid_adjoint(S, ix, iy, false, s, us);
+                         if (water) c.ub_w[n] = grid_adjoint(S, ix, iy, true, w, uw);
+                         if (TURN) {
+                             grid_velocity(c, S, n, ix, iy, solid_prev, water_prev, ps, pw);
+                             if (solid_prev) c.ub_s_prev[n] = zero;
+                             if (water_prev) c.ub_w_prev[n] = zero;
+                         }
+                     });
 }
 
 // Loss sum |x - target|^2 per scene (one atomic per warp whose particles
@@ -593,31 +618,28 @@ __global__ void __launch_bounds__(ADJ_THREADS) k_adj_loss(AdjCtx c)
     }
 }
 
-// The G2P adjoint of one substep: from the adjoints of the substep's outputs
-// (x, v, C, F) to the node-velocity adjoints (scattered) and the G2P parts of
+// A particle's adjoints of a state.
+struct StateAdjoint {
+    float2 x, v;
+    float4 C, F;
+};
+
+// The G2P adjoint of one particle: from the adjoints of the substep's outputs
+// to the node-velocity adjoints (added to ub_s / ub_w) and the G2P parts of
 // the input position and F adjoints.
-__global__ void __launch_bounds__(ADJ_THREADS, 3) k_adj_g2p_bwd(AdjCtx c)
+__device__ __forceinline__ void g2p_adjoint(const AdjCtx &c, uint32_t i, uint32_t tag, float2 x, float4 F0,
+                                            const StateAdjoint &o, float4 *ub_s, float4 *ub_w)
 {
-    // this thread's stencil node velocities and liquid sums from the forward
-    // recompute, read again by the adjoint's scatter
-    __shared__ float2 s_u[9][ADJ_THREADS];
-    __shared__ float2 s_mv[9][ADJ_THREADS];
-    follow();
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= c.n) return;
-    const uint32_t tag = c.tag[i];
     const AdjScene &S = c.scenes[tag >> 1];
     const bool liquid = (tag & 1u) != 0u;
-    const float2 x = c.in.x[i];
-    const float4 F0 = c.in.F[i];
     AdjStencil st;
     G2pFwd g;
-    if (!adj_stencil(S, x, st) || !g2p_forward<true>(c, S, liquid, st, x, F0, g, s_u, s_mv)) {
+    if (!adj_stencil(S, x, st) || !g2p_forward(c, S, liquid, st, x, F0, g)) {
         adj_fail(c, ADJ_ERR_NONFINITE);
         return;
     }
-    const float2 xbo = c.xb_next[i], vbo = c.vb_next[i];
-    const float4 Cbo = c.Cb_next[i], Fbo = c.Fb_next[i];
+    const float2 xbo = o.x, vbo = o.v;
+    const float4 Cbo = o.C, Fbo = o.F;
     // confinement: a clamped axis passes no gradient
     const float2 cxa = confine_axis(g.xn.x, g.vp.x, S.domain_w);
     const float2 cya = confine_axis(g.xn.y, g.vp.y, S.domain_h);
@@ -677,20 +699,21 @@ __global__ void __launch_bounds__(ADJ_THREADS, 3) k_adj_g2p_bwd(AdjCtx c)
         for (int ox = 0; ox < 3; ++ox) {
             const float w = st.wx[ox] * st.wy[oy];
             const float dpx = ((float)ox - st.fx) * S.dx;
-            const float2 u = s_u[oy * 3 + ox][threadIdx.x];
-            const float2 mv = s_mv[oy * 3 + ox][threadIdx.x];  // liquid mass and volume
+            // the node velocity, liquid mass and volume once more
+            const uint32_t n = adj_node(S, st.bx + ox, st.by + oy);
+            const float4 gw = liquid ? c.gv_w[n] : make_float4(c.gv_s[n].x, c.gv_s[n].y, 0.f, 0.f);
+            const float2 u = make_float2(gw.x, gw.y);
             // node velocity adjoint: w vpb + w Bb dp
             const float ubx = w * (vpb.x + Bb.x * dpx + Bb.y * dpy);
             const float uby = w * (vpb.y + Bb.z * dpx + Bb.w * dpy);
-            const uint32_t n = adj_node(S, st.bx + ox, st.by + oy);
             if (liquid)
-                atomicAdd(&c.ub_w[n], make_float4(ubx, uby, w * pm_b, w * pv_b));
+                atomicAdd(&ub_w[n], make_float4(ubx, uby, w * pm_b, w * pv_b));
             else
-                atomicAdd(reinterpret_cast<float2 *>(&c.ub_s[n]), make_float2(ubx, uby));
+                atomicAdd(reinterpret_cast<float2 *>(&ub_s[n]), make_float2(ubx, uby));
             // d/dx of w: (dwx wy, wx dwy) / dx
             const float gwx = st.dwx[ox] * st.wy[oy] * S.inv_dx, gwy = st.wx[ox] * st.dwy[oy] * S.inv_dx;
             float sval = u.x * (vpb.x + Bb.x * dpx + Bb.y * dpy) + u.y * (vpb.y + Bb.z * dpx + Bb.w * dpy);
-            if (liquid) sval += pm_b * mv.x + pv_b * mv.y;
+            if (liquid) sval += pm_b * gw.z + pv_b * gw.w;
             // dp = (k - f) dx: d/dx = -1 per axis
             xb.x += gwx * sval - w * (u.x * Bb.x + u.y * Bb.z);
             xb.y += gwy * sval - w * (u.x * Bb.y + u.y * Bb.w);
@@ -698,6 +721,17 @@ __global__ void __launch_bounds__(ADJ_THREADS, 3) k_adj_g2p_bwd(AdjCtx c)
     }
     c.xg[i] = xb;
     c.Fg[i] = Fg;
+}
+
+// The G2P adjoint of the last substep of a segment (the others' comes with
+// the P2G adjoint of the substep after them).
+__global__ void __launch_bounds__(ADJ_THREADS, 3) k_adj_g2p_bwd(AdjCtx c)
+{
+    follow();
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= c.n) return;
+    const StateAdjoint o{c.xb_next[i], c.vb_next[i], c.Cb_next[i], c.Fb_next[i]};
+    g2p_adjoint(c, i, c.tag[i], c.in.x[i], c.in.F[i], o, c.ub_s, c.ub_w);
 }
 
 // Sum of a value over the lanes of a warp whose particles all belong to one
@@ -726,19 +760,27 @@ __device__ __forceinline__ void add_param_grads(double *grad, uint32_t scene, fl
     }
 }
 
-// The grid-update and P2G adjoint of one substep, fused: each particle
-// gathers, for its nine nodes, the adjoints of the node sums (from the node
-// velocity adjoints and the sums, finishGridVelocity and the wall factors
-// reversed), then reverses its own P2G contribution and stress; adds the G2P
-// parts; writes the adjoints of the substep's inputs and the parameter
-// gradients.
-__global__ void __launch_bounds__(ADJ_THREADS, 4) k_adj_p2g_bwd(AdjCtx c)
+// The P2G adjoint of one substep: each particle gathers, for its nine nodes,
+// the adjoints of the node sums, then reverses its own P2G contribution and
+// stress, adds the G2P parts, and has the adjoints of the substep's inputs and the
+// parameter gradients.  TURN: those inputs are the outputs of the substep before,
+// whose state is c.out and whose G2P adjoint follows at once; else they
+// are written.  Bound by the latency of the gathers and by L1: the G2P
+// adjoint reads its nodes' velocities a second time rather than keep them (shared
+// memory for 36 KB a CTA took L1's room and a CTA per SM: per million particles
+// 110.8 us, 96.8 without it, 91.8 with 64 registers for a fourth CTA; as two kernels
+// 47 + 73).  Where the CTAs are at most two per SM, four cannot meet: the instance
+// with room for all registers (1,024 particles: 7.6 -> 6.9 us, 65,536: 10.1 -> 9.6;
+// above that line it loses, 98,304: 12.6 against 15.9).
+template <bool TURN, int CTAS>
+__global__ void __launch_bounds__(ADJ_THREADS, CTAS) k_adj_p2g_bwd(AdjCtx c)
 {
     follow();
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     const bool valid = i < c.n;
     const uint32_t tag = valid ? c.tag[i] : 0u, scene = tag >> 1;
     float3 pg = make_float3(0.f, 0.f, 0.f);
+    StateAdjoint a{};
     bool ok = valid;
     if (valid) {
         const AdjScene &S = c.scenes[scene];
@@ -787,16 +829,22 @@ __global__ void __launch_bounds__(ADJ_THREADS, 4) k_adj_p2g_bwd(AdjCtx c)
             float4 Fb = c.Fg[i];
             if (liquid) Fb = axpy4(vliq_b * vol, cofactor(F), Fb);
             pg = stress_adjoint(S, liquid, F, p.det, sb, Fb);
-            c.xb[i] = xb;
-            c.vb[i] = vb;
-            c.Cb[i] = Cb;
-            c.Fb[i] = Fb;
+            a = StateAdjoint{xb, vb, Cb, Fb};
             if (!finite2(xb) || !finite2(vb) || !finite4(Cb) || !finite4(Fb)) adj_fail(c, ADJ_ERR_NONFINITE);
         } else {
             adj_fail(c, ADJ_ERR_NONFINITE);
         }
     }
     add_param_grads(c.param_grad, scene, pg, ok);
+    if (!ok) return;
+    if constexpr (TURN) {
+        g2p_adjoint(c, i, tag, c.out.x[i], c.out.F[i], a, c.ub_s_prev, c.ub_w_prev);
+    } else {
+        c.xb[i] = a.x;
+        c.vb[i] = a.v;
+        c.Cb[i] = a.C;
+        c.Fb[i] = a.F;
+    }
 }
 
 // ----------------------------------------------------------------- host ---
@@ -822,8 +870,9 @@ struct mpm_adjoint {
     size_t mark_count = 0;
     uint32_t *tile_scene = nullptr;             // per tile
     uint32_t n_tiles = 0, tile_ctas = 1;
+    unsigned sms = 1;
     float2 *xb[2]{}, *vb[2]{}, *xg = nullptr;
-    float4 *Cb[2]{}, *Fb[2]{}, *Fg = nullptr, *ub_w = nullptr, *ub_s = nullptr;
+    float4 *Cb[2]{}, *Fb[2]{}, *Fg = nullptr, *ub_w[2]{}, *ub_s[2]{};
     float2 *gv_s = nullptr;  // node velocities of the substep at hand
     float4 *gv_w = nullptr;
     // loss per scene, the status word (in 8 bytes), three parameter gradients per scene
@@ -877,7 +926,7 @@ void free_engine(mpm_adjoint *a)
     for (float4 *p : a->tape_s) cudaFree(p);
     for (float4 *p : a->tape_w) cudaFree(p);
     void *ptrs[] = {a->mark,  a->tile_scene, a->d_scenes, a->tag,   a->vol,   a->sum_s, a->sum_w,
-                    a->xb[0], a->xb[1],      a->vb[0],    a->vb[1], a->xg,    a->ub_s,  a->ub_w, a->Cb[0], a->Cb[1],
+                    a->xb[0], a->xb[1],      a->vb[0],    a->vb[1], a->xg,    a->ub_s[0], a->ub_s[1], a->ub_w[0], a->ub_w[1], a->Cb[0], a->Cb[1],
                     a->Fb[0], a->Fb[1],      a->Fg,       a->gv_s,  a->gv_w,  a->results, a->target, a->final_x};
     for (void *p : ptrs)
         if (p) cudaFree(p);
@@ -926,8 +975,8 @@ AdjCtx make_adj_ctx(mpm_adjoint *a, const AdjState &in, const AdjState &out, flo
     c.Fb = a->Fb[1 - adj];
     c.xg = a->xg;
     c.Fg = a->Fg;
-    c.ub_s = a->ub_s;
-    c.ub_w = a->ub_w;
+    c.ub_s = a->ub_s[0];
+    c.ub_w = a->ub_w[0];
     c.gv_s = a->gv_s;
     c.gv_w = a->gv_w;
     c.param_grad = a->param_grad();
@@ -1137,8 +1186,10 @@ int mpma_create(const mpm_config *configs, uint32_t scene_count, const uint32_t 
     }
     ADJ_ALLOC(a->xg, n);
     ADJ_ALLOC(a->Fg, n);
-    ADJ_ALLOC(a->ub_s, nodes);
-    ADJ_ALLOC(a->ub_w, nodes);
+    for (int b = 0; b < 2; ++b) {
+        ADJ_ALLOC(a->ub_s[b], nodes);
+        ADJ_ALLOC(a->ub_w[b], nodes);
+    }
     ADJ_ALLOC(a->gv_s, nodes);
     ADJ_ALLOC(a->gv_w, nodes);
     ADJ_ALLOC(a->results, 4 * (size_t)scene_count + 1);
@@ -1150,6 +1201,7 @@ int mpma_create(const mpm_config *configs, uint32_t scene_count, const uint32_t 
     int sms = 1;
     if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess)
         return fail(err(MPM_ERR_CUDA, "device query failed"));
+    a->sms = (unsigned)sms;
     a->tile_ctas = (uint32_t)sms * 8u;  // 2048 threads per SM
     bool ok = cudaMemcpy(a->d_scenes, scenes.data(), scene_count * sizeof(AdjScene), cudaMemcpyHostToDevice) == cudaSuccess;
     ok = ok && cudaMemcpy(a->tag, tag.data(), n * sizeof(uint32_t), cudaMemcpyHostToDevice) == cudaSuccess;
@@ -1305,16 +1357,33 @@ int mpma_backward(mpm_adjoint *a, float *grad_velocities, double *grad_parameter
             ADJ_TRY(run_substeps(a, start, len, state, true, true, false, false));
             a->tape_segment = seg;
         }
-        for (int j = (int)len - 1; j >= 0; --j) {
-            const uint32_t k = start + (uint32_t)j;
-            const AdjCtx c = make_adj_ctx(a, state(k), state(k), a->tape_s[j], a->tape_w[j], adj);
-            over_tiles(a, k_adj_grid_fwd<false>, c, tile_scenes(a), tile_marks(a, k), a->n_tiles, (float4 *)nullptr,
-                       (float4 *)nullptr);
-            over_particles(a, k_adj_g2p_bwd, c);
-            over_tiles(a, k_adj_grid_bwd, c, tile_scenes(a), tile_marks(a, k), a->n_tiles);
-            over_particles(a, k_adj_p2g_bwd, c);
-            adj = 1 - adj;
+        // substep by substep from the segment's last; node adjoints of one
+        // substep in one pair of buffers, of the one before it in the other
+        int ub = 0;
+        const auto substep = [&](uint32_t k) {
+            const uint32_t j = k - start;
+            AdjCtx c = make_adj_ctx(a, state(k), j > 0u ? state(k - 1u) : state(k), a->tape_s[j], a->tape_w[j], adj);
+            c.ub_s = a->ub_s[ub], c.ub_w = a->ub_w[ub];
+            c.ub_s_prev = a->ub_s[1 - ub], c.ub_w_prev = a->ub_w[1 - ub];
+            return c;
+        };
+        const uint32_t last = start + len - 1u;
+        over_tiles(a, k_adj_grid_fwd<false>, substep(last), tile_scenes(a), tile_marks(a, last), a->n_tiles, (float4 *)nullptr,
+                   (float4 *)nullptr);
+        over_particles(a, k_adj_g2p_bwd, substep(last));
+        for (uint32_t k = last; k > start; --k) {
+            over_tiles(a, k_adj_grid_bwd<true>, substep(k), tile_scenes(a), tile_marks(a, k), tile_marks(a, k - 1u), a->n_tiles,
+                       (const float4 *)a->tape_s[k - 1u - start], (const float4 *)a->tape_w[k - 1u - start]);
+            if (blocks(a->n) <= 2u * a->sms)
+                over_particles(a, k_adj_p2g_bwd<true, 2>, substep(k));
+            else
+                over_particles(a, k_adj_p2g_bwd<true, 4>, substep(k));
+            ub = 1 - ub;
         }
+        over_tiles(a, k_adj_grid_bwd<false>, substep(start), tile_scenes(a), tile_marks(a, start), (const uint8_t *)nullptr,
+                   a->n_tiles, (const float4 *)nullptr, (const float4 *)nullptr);
+        over_particles(a, k_adj_p2g_bwd<false, 4>, substep(start));
+        adj = 1 - adj;
         ADJ_TRY(cudaGetLastError());
     }
     ADJ_TRY(cudaEventRecord(a->ev[3], a->stream));

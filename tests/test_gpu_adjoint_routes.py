@@ -55,3 +55,30 @@ def test_one_material_and_a_reused_engine(steps, every):
         assert _near(again[1], gv) and _near(again[2], gp)
     finally:
         both.dispose()
+
+
+@pytest.mark.parametrize("every", [1, 3, 8])
+def test_a_batch_above_two_ctas_per_sm_has_the_gradients_of_its_scenes(every):
+    """Turning from a substep to the one before takes another instance of the
+    kernel where 148 SMs hold more than two CTAs of 256 particles each; every 1
+    turns nowhere."""
+    scenes = create_adjoint_scenes(8, seed=5, water_columns=96, water_rows=98, solid_side=20, cells=128)
+    assert sum(len(p) for p, _, _ in scenes) > 2 * 148 * 256
+    dts = [float(np.float32(fixed_cfl_dt(p, c, 90.0, 0.05))) for p, c, _ in scenes]
+    batch = create_mpm_adjoint_engine([(p, c) for p, c, _ in scenes], ADJOINT_GRAVITY)
+    try:
+        losses = batch.forward(8, dts, np.concatenate([t for _, _, t in scenes]), checkpoint_every=every)
+        gv, gp = batch.backward()
+    finally:
+        batch.dispose()
+    first = 0
+    for k, (p, c, t) in enumerate(scenes):
+        if k in (0, 7):
+            alone = create_mpm_adjoint_engine([(p, c)], ADJOINT_GRAVITY)
+            try:
+                loss, own_gv, own_gp = _gradients(alone, 8, every, dts[k], t)
+            finally:
+                alone.dispose()
+            assert abs(losses[k] - loss[0]) <= 1e-4 * loss[0]
+            assert _near(gv[first:first + len(p)], own_gv) and _near(gp[k], own_gp[0])
+        first += len(p)
