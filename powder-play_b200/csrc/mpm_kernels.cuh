@@ -153,7 +153,8 @@ constexpr int VOL_Y = RING_Y + 2;
 constexpr int G2P_THREADS = 256;
 constexpr uint32_t G2P_MAX_PARTS = 4;      // CTAs that may share a tile in G2P
 constexpr int FIELD_BODY_CHUNK = TILE_NODES;  // bodies staged per pass of k_triangle_field
-constexpr int BODY_THREADS = 64;              // k_body_impulses: one CTA per body
+constexpr int BODY_THREADS = 64;              // k_body_contacts: one CTA per body,
+constexpr int PAIRS_PER_THREAD = 4;           // and body pairs per thread of its other CTAs
 constexpr uint32_t PAIR_CACHE_BODIES = 2048;  // bodies up to which pair contacts are cached
 constexpr int BONDED_TRIANGLE_SOLVER_ITERATIONS = 2;
 constexpr int G2P_STAGE = 2 * G2P_THREADS;  // particles of a tile staged at once
@@ -221,10 +222,7 @@ __global__ void k_end_batch(Ctx c, uint32_t total_steps, uint32_t measure_speed)
 __global__ void k_begin_batch(Ctx c, uint32_t reset_progress);
 // bodies and fracture
 __global__ void k_triangle_field(Ctx c);
-__global__ void k_body_impulses(Ctx c);
-__global__ void k_body_bonded(Ctx c);
-__global__ void k_body_states(Ctx c);
-__global__ void k_body_pairs(Ctx c);
+__global__ void k_body_contacts(Ctx c, uint32_t body_ctas);
 __global__ void k_body_apply(Ctx c);
 __global__ void k_validate_cfl(Ctx c);
 __global__ void k_fracture_bonds(Ctx c);

@@ -372,18 +372,18 @@ void enqueue_cell_sort(mpm_solver *s, const Ctx &c)
 }
 
 // The passes after G2P for bonded-triangle bodies and fracture bonds, in the
-// reference's order (solver.ts:1505-1562): contact impulses, bonded edges,
-// contact states, pair contacts, the CFL check, fracture; then the tile
-// counts and P2G records of the particles those passes moved.
+// reference's order (solver.ts:1505-1562): contact impulses, bonded edges and
+// contact states with the pair contacts in one launch, their impulses, the CFL
+// check, fracture; then the tile counts and P2G records of the particles those
+// passes moved.
 void enqueue_bodies(mpm_solver *s, const Ctx &c)
 {
     const uint32_t nb = s->n_bodies;
     if (nb) {
         const unsigned bb = blocks_for(nb, 64);
-        launch(s, k_body_impulses, dim3(std::min(nb, 1024u)), dim3(BODY_THREADS), 0, c);
-        launch(s, k_body_bonded, dim3(bb), dim3(64), 0, c);
-        launch(s, k_body_states, dim3(bb), dim3(64), 0, c);
-        if (s->pair_cache) launch(s, k_body_pairs, dim3(blocks_for(nb * nb, 256)), dim3(256), 0, c);
+        const unsigned body_ctas = std::min(nb, 1024u);
+        const unsigned pair_ctas = s->pair_cache ? blocks_for(nb * nb, BODY_THREADS * PAIRS_PER_THREAD) : 0u;
+        launch(s, k_body_contacts, dim3(body_ctas + pair_ctas), dim3(BODY_THREADS), 0, c, (uint32_t)body_ctas);
         launch(s, k_body_apply, dim3(bb), dim3(64), 0, c);
         // captured graphs serve batches with and without a CFL guard: the
         // kernel reads the batch's flag from the device parameters
@@ -391,7 +391,8 @@ void enqueue_bodies(mpm_solver *s, const Ctx &c)
     }
     if (s->n_bonds) {
         launch(s, k_fracture_bonds, dim3(blocks_for(s->n_bonds, 64)), dim3(64), 0, c);
-        if (s->n_endpoints) launch(s, k_fracture_damage, dim3(blocks_for(s->n_endpoints, 64)), dim3(64), 0, c);
+        // (of the default path with k_body_finish)
+        if (s->n_endpoints && !s->gather()) launch(s, k_fracture_damage, dim3(blocks_for(s->n_endpoints, 64)), dim3(64), 0, c);
     }
     if (s->gather() && s->n_tracked) launch(s, k_body_finish, dim3(blocks_for(s->n_tracked, 64)), dim3(64), 0, c);
 }
@@ -1133,11 +1134,10 @@ int create_impl(const mpm_config *configs, uint32_t n_scenes, const uint32_t *co
             const uint32_t marker = f2u(packed[(size_t)i * MPM_PARTICLE_WORDS + 19]);
             const bool endpoint = bond_count > 0 && topology[i + 1] > topology[i];
             if (endpoint) endpoints.push_back(i);
-            if (marker != 0u || endpoint) {
-                flag[i] = 1u;
-                tracked.push_back(i);
-            }
+            else if (marker != 0u) tracked.push_back(i);
+            if (marker != 0u || endpoint) flag[i] = 1u;
         }
+        tracked.insert(tracked.begin(), endpoints.begin(), endpoints.end());  // the endpoints first
         s->n_tracked = (uint32_t)tracked.size();
         s->n_endpoints = (uint32_t)endpoints.size();
         ALLOC(s->track_flag, cap);
