@@ -253,34 +253,34 @@ __device__ __forceinline__ float2 confine_axis(float next, float vel, float maxi
     return make_float2(next, vel);
 }
 
-// applyWallCushion / applyWallTangentialFriction: shaders.ts:1438-1457
+// applyWallCushion / applyWallTangentialFriction (shaders.ts:1438-1457) as the
+// factors of a velocity component near the walls of an axis of `extent` cells.
 // (dist / cushion clamped to [0, 1] is exactly 1 once dist >= cushion, so
 // nodes away from the walls skip the division.)
-__device__ __forceinline__ float wall_cushion(float vel, int coord, int extent)
+__device__ __forceinline__ float wall_cushion_width(int extent) { return fminf(WALL_CUSHION_CELLS, (float)extent / 4.0f); }
+
+__device__ __forceinline__ float wall_cushion_factor(float vel, int coord, int extent, float cushion)
 {
-    float cushion = fminf(WALL_CUSHION_CELLS, (float)extent / 4.0f);
-    float dist = vel < 0.0f ? (float)coord : (float)(extent - coord);
-    if (dist >= cushion) return vel;
-    return vel * fminf(fmaxf(dist / cushion, 0.0f), 1.0f);
+    const float dist = vel < 0.0f ? (float)coord : (float)(extent - coord);
+    return dist >= cushion ? 1.0f : fminf(fmaxf(dist / cushion, 0.0f), 1.0f);
+}
+
+// The factor of the components along the walls of the axis, whatever they are.
+__device__ __forceinline__ float wall_friction_factor(int coord, int extent, float cushion, float friction)
+{
+    const float dist = fmaxf(0.0f, fminf((float)coord, (float)(extent - coord)));
+    if (friction <= 0.0f || dist >= cushion) return 1.0f;
+    const float influence = 1.0f - fminf(fmaxf(dist / cushion, 0.0f), 1.0f);
+    return 1.0f - friction * influence;
 }
 
 // Whether every coordinate in [lo, hi] lies at least the cushion from both
-// walls of an axis of `extent` cells: wall_cushion and wall_friction then
-// return the velocity they are given, for either sign.
+// walls of an axis of `extent` cells: both factors are then 1, for either
+// sign.
 __device__ __forceinline__ bool beyond_wall_cushion(int lo, int hi, int extent)
 {
-    const float cushion = fminf(WALL_CUSHION_CELLS, (float)extent / 4.0f);
+    const float cushion = wall_cushion_width(extent);
     return (float)lo >= cushion && (float)(extent - hi) >= cushion;
-}
-
-__device__ __forceinline__ float wall_friction(float vel, int coord, int extent, float friction)
-{
-    if (friction <= 0.0f) return vel;
-    float dist = fmaxf(0.0f, fminf((float)coord, (float)(extent - coord)));
-    float cushion = fminf(WALL_CUSHION_CELLS, (float)extent / 4.0f);
-    if (dist >= cushion) return vel;
-    float influence = 1.0f - fminf(fmaxf(dist / cushion, 0.0f), 1.0f);
-    return vel * (1.0f - friction * influence);
 }
 
 // pow as WGSL specifies it: its accuracy is inherited from

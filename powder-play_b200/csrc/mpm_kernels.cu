@@ -708,24 +708,21 @@ __device__ __forceinline__ bool node_velocity(const Ctx &c, uint32_t n, int x, i
         return false;
     }
     if (near_wall) {
+        // the friction factors are the node's; a channel without mass has no
+        // velocity: water alone takes four divisions where one function call per
+        // component took eight and more (a substep of the 1,600-particle tank 20.3
+        // -> 19.3 us, of 20,011 21.7 -> 21.1)
         const int cx = (int)P.cells_x, cy = (int)P.cells_y;
-        const float fr = P.wall_friction;
-        if (!LIQ) {
-            vs.x = wall_cushion(vs.x, x, cx);
-            vs.y = wall_cushion(vs.y, y, cy);
-        }
-        vw.x = wall_cushion(vw.x, x, cx);
-        vw.y = wall_cushion(vw.y, y, cy);
-        vo.x = wall_cushion(vo.x, x, cx);
-        vo.y = wall_cushion(vo.y, y, cy);
-        if (!LIQ) {
-            vs.x = wall_friction(vs.x, y, cy, fr);
-            vs.y = wall_friction(vs.y, x, cx, fr);
-        }
-        vw.x = wall_friction(vw.x, y, cy, fr);
-        vw.y = wall_friction(vw.y, x, cx, fr);
-        vo.x = wall_friction(vo.x, y, cy, fr);
-        vo.y = wall_friction(vo.y, x, cx, fr);
+        const float width_x = wall_cushion_width(cx), width_y = wall_cushion_width(cy);
+        const float along_x = wall_friction_factor(y, cy, width_y, P.wall_friction);
+        const float along_y = wall_friction_factor(x, cx, width_x, P.wall_friction);
+        auto wall = [&](float &vx, float &vy) {
+            vx = vx * wall_cushion_factor(vx, x, cx, width_x) * along_x;
+            vy = vy * wall_cushion_factor(vy, y, cy, width_y) * along_y;
+        };
+        if (!LIQ && S.x > 0.f) wall(vs.x, vs.y);
+        if (W.x > 0.f) wall(vw.x, vw.y);
+        if (O.x > 0.f) wall(vo.x, vo.y);
     }
     const float lm = W.x + O.x, lv = W.w + O.w;
     out.vs = vs;
