@@ -837,7 +837,8 @@ def run_b200(args):
         "gpu_launches": gpu_launches,
     }
     if args.p2g == "fixed" and "k_prepare_scatter" in prof:
-        # the fixed-point scatter's int32 atomics: 9 nodes x 4 words per
+        # the fixed-point scatter's int32 contributions, summed in shared
+        # memory first where a CTA's nodes lie together: 9 nodes x 4 words per
         # liquid particle (mass, momentum, volume), 9 x 3 per solid one
         packed, _ = solver.read_particles_packed()
         model = packed[:, 13].view(np.uint32)

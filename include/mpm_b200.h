@@ -256,9 +256,9 @@ int mpm_get_launch_shape(mpm_solver *solver, uint32_t *p2g_ctas, uint32_t *g2p_c
  * parameters (the whole graph, device time) for each candidate variant and
  * keeps the fastest: for each P2G stage capacity (640, 384), the one-launch
  * substep over persistent grids of 1 .. co-resident CTAs per SM, and the
- * four-launch substep over its P2G grids, then its G2P grids with the best
+ * substep in separate launches over its P2G grids, then its G2P grids with the best
  * P2G, then both ways of handing prepareParticle's results to P2G.  Restores the particle state and counters it started from.  Returns
- * the chosen four-launch grids (mpm_get_substep_variant gives the rest) and
+ * the chosen P2G and G2P grids (mpm_get_substep_variant gives the rest) and
  * the best milliseconds per substep.  Needs one submitted batch.  Blocks. */
 int mpm_autotune(mpm_solver *solver, uint32_t substeps, uint32_t *p2g_ctas, uint32_t *g2p_ctas, double *best_ms);
 
@@ -266,7 +266,7 @@ int mpm_autotune(mpm_solver *solver, uint32_t substeps, uint32_t *p2g_ctas, uint
  * whose substep is a sequence of WebGPU compute passes).  `fused` 1 runs each
  * substep as ONE cooperative launch of persistent CTAs (tile allocation,
  * bucketing, P2G, grid update + G2P, with grid barriers between them), 0 as
- * four launches; `stage_capacity` is the P2G stage (640 or 384 particles;
+ * separate launches; `stage_capacity` is the P2G stage (640 or 384 particles;
  * 0 keeps it); `substep_ctas` the one-launch form's persistent grid (0 keeps
  * it; at most the CTAs that fit on the GPU at once); `liquid_kernels` 1 lets
  * G2P run its instantiation compiled for water and oil only whenever every
@@ -276,7 +276,7 @@ int mpm_autotune(mpm_solver *solver, uint32_t substeps, uint32_t *p2g_ctas, uint
  * next P2G, 0 has P2G prepare each particle from its state, 2 picks by the
  * materials (records unless every material is a liquid with the linear EOS;
  * the one-launch form always prepares in P2G).  Solvers with bonded bodies or
- * fracture bonds always take four launches and the general G2P.  Results do
+ * fracture bonds always take separate launches and the general G2P.  Results do
  * not depend on `fused`, the grids, `liquid_kernels` or `p2g_records` (the
  * same arithmetic); the stage capacity changes only the rounding of tiles
  * holding more particles than it.  mpm_get_substep_variant reports whether

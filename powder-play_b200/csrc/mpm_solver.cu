@@ -147,7 +147,7 @@ struct mpm_solver {
     unsigned sms = 1;
     unsigned p2g_ctas = 1, g2p_ctas = 1;  // persistent grids of the default path's P2G and G2P kernels
     // the default path's substep variant: one cooperative launch (k_substep)
-    // or four launches, the P2G stage capacity, k_substep's persistent grid
+    // or separate launches, the P2G stage capacity, k_substep's persistent grid
     // and the most CTAs of it that fit on the GPU at once
     bool fused = false;
     int stage_cap = STAGE_CAP;
@@ -1711,7 +1711,7 @@ int mpm_autotune(mpm_solver *s, uint32_t substeps, uint32_t *p2g_ctas, uint32_t 
     const bool guarded = s->h_params[0].cfl_enabled != 0u;
     // one candidate: every setting of the variant, timed over `substeps`
     // real substeps from the saved state (the whole graph, no events between
-    // kernels, so the four-launch and one-launch forms compare fairly)
+    // kernels, so the separate and one-launch forms compare fairly)
     struct Candidate {
         bool fused;
         int cap;
@@ -1738,7 +1738,7 @@ int mpm_autotune(mpm_solver *s, uint32_t substeps, uint32_t *p2g_ctas, uint32_t 
         if (rc == MPM_OK && ms < best_ms_total) best_ms_total = ms, best = v;
     };
     // the stage variants; for each, the one-launch form over persistent grids
-    // of 1 .. (co-resident limit) CTAs per SM, and the four-launch form over
+    // of 1 .. (co-resident limit) CTAs per SM, and the separate launches over
     // its P2G grids, then its G2P grids with the best P2G (a grid of one CTA
     // per tile is not a candidate: it pays for every tile of every scene in
     // substeps that list few)

@@ -326,7 +326,7 @@ class MpmBatchedGpuSolver:
 
     def substep_variant(self) -> dict:
         """How the default path runs a substep: `fused` (one cooperative launch
-        of persistent CTAs, else four launches), the P2G stage capacity, the
+        of persistent CTAs, else separate launches), the P2G stage capacity, the
         one-launch form's persistent grid and its co-resident limit, whether
         G2P runs its water-and-oil instantiation and whether G2P writes the
         next P2G's records."""
