@@ -1031,24 +1031,32 @@ __global__ void k_tile_scatter(Ctx c)
 // more, a round then takes its chain of dependent instructions).
 // The last CTA to have read whether the scene runs starts the substep
 // (begin_substep).  What it costs is latency: the counts, keys and ranks come
-// in together, then the scan, then the stores; a substep of 1,600 particles
-// fell from 21.8 to 21.2 us against the two kernels, one of 150,000 from 31.0 to
-// 30.5 us.
-__global__ void __launch_bounds__(BUCKET_THREADS) k_tile_bucket(Ctx c)
+// in together, then the scan, then the stores.  A CTA has as few threads as
+// its barriers, scan and start are short with, of TILES tiles each: against 1,024
+// threads of 4 tiles a substep of 1,600 particles fell from 19.4 to 18.6 us, of
+// 20,011 (325 tiles) from 21.1 to 19.6, of 150,002 (1,056 tiles, 256 threads of
+// 8) from 29.2 to 28.2; 128 threads of 8 tiles 20.3 and 256 of 16 29.2 there
+// (two kernels instead of one: 0.6 us more).
+template <int THREADS, int TILES>
+__global__ void __launch_bounds__(THREADS) k_tile_bucket(Ctx c)
 {
     follow();
-    __shared__ uint32_t s_first[BUCKET_TILES];  // first bucket entry per tile
+    __shared__ uint32_t s_first[TILES * THREADS];  // first bucket entry per tile
+    __shared__ unsigned long long s_warp[THREADS / 32];
     __shared__ bool s_runs;
     const uint32_t n_tiles = c.P->scene_tiles;
-    const uint32_t t0 = threadIdx.x * 4u;
-    const uint32_t i = (blockIdx.x * BUCKET_THREADS + threadIdx.x) * 4u;
-    uint32_t v[4], key[4], rank[4];
-    if (t0 + 4u <= n_tiles) {
-        const uint4 a = __ldcg(reinterpret_cast<const uint4 *>(c.tile_count + t0));
-        v[0] = a.x, v[1] = a.y, v[2] = a.z, v[3] = a.w;
-    } else {
+    const uint32_t t0 = threadIdx.x * TILES;
+    const uint32_t i = (blockIdx.x * THREADS + threadIdx.x) * 4u;
+    uint32_t v[TILES], key[4], rank[4];
 #pragma unroll
-        for (int k = 0; k < 4; ++k) v[k] = t0 + k < n_tiles ? __ldcg(c.tile_count + t0 + k) : 0u;
+    for (uint32_t t = 0; t < TILES; t += 4u) {
+        if (t0 + t + 4u <= n_tiles) {
+            const uint4 a = __ldcg(reinterpret_cast<const uint4 *>(c.tile_count + t0 + t));
+            v[t] = a.x, v[t + 1u] = a.y, v[t + 2u] = a.z, v[t + 3u] = a.w;
+        } else {
+#pragma unroll
+            for (uint32_t k = t; k < t + 4u; ++k) v[k] = t0 + k < n_tiles ? __ldcg(c.tile_count + t0 + k) : 0u;
+        }
     }
     if (i + 4u <= c.n) {
         const uint4 a = __ldcg(reinterpret_cast<const uint4 *>(c.keys + i));
@@ -1067,18 +1075,37 @@ __global__ void __launch_bounds__(BUCKET_THREADS) k_tile_bucket(Ctx c)
     // particles in the high word; listed tiles and G2P items (at most 4096 and
     // 16384) in the low and high halves of the low word
     unsigned long long mine = 0ull, total;
-    uint32_t parts[4];
+    uint32_t parts[TILES];
 #pragma unroll
-    for (int k = 0; k < 4; ++k) {
+    for (int k = 0; k < TILES; ++k) {
         parts[k] = c.divided ? min((v[k] + G2P_THREADS - 1u) / G2P_THREADS, G2P_MAX_PARTS) : (v[k] != 0u ? 1u : 0u);
         mine += ((unsigned long long)v[k] << 32) | (parts[k] << 16) | (v[k] != 0u ? 1u : 0u);
     }
-    const unsigned long long offset = block_exclusive_scan<BUCKET_THREADS, unsigned long long>(mine, total);
+    // the scan over the CTA with one barrier: every warp adds up the warps'
+    // totals itself
+    const uint32_t lane = threadIdx.x % 32u, warp = threadIdx.x / 32u;
+    unsigned long long upto = mine;
+#pragma unroll
+    for (uint32_t o = 1u; o < 32u; o <<= 1) {
+        const unsigned long long n = __shfl_up_sync(0xffffffffu, upto, o);
+        if (lane >= o) upto += n;
+    }
+    if (lane == 31u) s_warp[warp] = upto;
+    __syncthreads();
+    unsigned long long warps = lane < THREADS / 32u ? s_warp[lane] : 0ull;
+    const unsigned long long own = warps;
+#pragma unroll
+    for (uint32_t o = 1u; o < THREADS / 32u; o <<= 1) {
+        const unsigned long long n = __shfl_up_sync(0xffffffffu, warps, o);
+        if (lane >= o) warps += n;
+    }
+    total = __shfl_sync(0xffffffffu, warps, THREADS / 32 - 1);
+    const unsigned long long offset = __shfl_sync(0xffffffffu, warps - own, (int)warp) + upto - mine;
     const bool runs = s_runs;
     uint32_t at = (uint32_t)(offset >> 32);
     uint32_t slot = (uint32_t)offset & 0xffffu, item = ((uint32_t)offset >> 16) & 0xffffu;
 #pragma unroll
-    for (int k = 0; k < 4; ++k) {
+    for (int k = 0; k < TILES; ++k) {
         s_first[t0 + k] = at;
         if (blockIdx.x == 0 && runs && v[k] != 0u) {
             c.active_tiles[slot++] = make_uint4(t0 + k, at, v[k], 0u);
@@ -3966,6 +3993,9 @@ __global__ void k_surface_decode(unsigned long long *acc, float2 *field, uint32_
 }
 
 // the instances the host launches
+template __global__ void k_tile_bucket<256, 4>(Ctx);
+template __global__ void k_tile_bucket<256, 8>(Ctx);
+template __global__ void k_tile_bucket<512, 8>(Ctx);
 // The trial deformation G2P computes (deformation_trial) for `n` given
 // (F, C) pairs: trial F, increment, determinant and substep count, or the
 // flags of a failed integration in `flags`.

@@ -132,8 +132,7 @@ constexpr int SCAN_CHUNK = SCAN_THREADS * SCAN_ITEMS;
 constexpr int SCAN_TOP_THREADS = 1024;
 constexpr int ALLOC_THREADS = 256;  // k_tile_alloc: 4 tiles per thread, 1024 per CTA
 constexpr int ALLOC_ITEMS = 4;
-constexpr int BUCKET_THREADS = 1024;  // k_tile_bucket: 4 tiles and 4 slots per thread
-constexpr uint32_t BUCKET_TILES = BUCKET_THREADS * 4;
+constexpr uint32_t BUCKET_TILES = 4096;  // tiles k_tile_bucket takes at most (512 threads of 8)
 constexpr uint32_t ALLOC_TILES = ALLOC_THREADS * ALLOC_ITEMS;
 
 // default P2G: the particles whose base node lies in one 16x8-node tile reach
@@ -194,6 +193,7 @@ __global__ void k_stable_rank(Ctx c);
 __global__ void k_tile_count(Ctx c);
 __global__ void k_tile_alloc(Ctx c);
 __global__ void k_tile_scatter(Ctx c);
+template <int THREADS, int TILES>
 __global__ void k_tile_bucket(Ctx c);
 // SCENES: the solver holds several scenes; CAP: particles staged at once;
 // ROLES: threads per cell of a tile; LIQ: every material is water or oil; REC: the records variant (P2G reads

@@ -537,7 +537,11 @@ void enqueue_substep(mpm_solver *s, int parity)
         mark(K_SUBSTEP);
     } else if (s->gather()) {
         if (buckets_at_once(s)) {
-            launch(s, k_tile_bucket, dim3(blocks_for((s->n + 3) / 4, BUCKET_THREADS)), dim3(BUCKET_THREADS), 0, c);
+            // the fewest threads whose tiles cover the scene's
+            const unsigned quads = (s->n + 3) / 4, n_tiles = s->scenes[0].tiles;
+            const unsigned threads = n_tiles <= 2048u ? 256u : 512u;
+            launch(s, n_tiles <= 1024u ? k_tile_bucket<256, 4> : (n_tiles <= 2048u ? k_tile_bucket<256, 8> : k_tile_bucket<512, 8>),
+                   dim3(blocks_for(quads, threads)), dim3(threads), 0, c);
             mark(K_TILE_BUCKET);
         } else {
             launch(s, k_tile_alloc, dim3(s->alloc_ctas), dim3(ALLOC_THREADS), 0, c);

@@ -60,3 +60,30 @@ def test_every_route_gives_the_one_launch_bits(n, cells_x, cells_y, spacing):
         finally:
             solver.dispose()
     assert np.array_equal(np.ascontiguousarray(runs[0]).view(np.uint32), np.ascontiguousarray(runs[1]).view(np.uint32))
+
+
+@pytest.mark.parametrize("cells_x, cells_y", [(509, 253), (510, 253), (509, 509), (509, 510)])
+def test_bucketing_at_each_number_of_tiles(cells_x, cells_y):
+    """1,024 tiles and 1,056, 2,048 and 2,080: the bucketing kernel's instances;
+    particles in the first and last tiles, few enough for one CTA and a second."""
+    for n in (1, 1_024, 1_025, 5_000):
+        rng = np.random.default_rng(n)
+        p = ParticleArrays.empty(n)
+        p.px[:], p.py[:] = rng.uniform(20, cells_x * 10 - 20, n), rng.uniform(20, cells_y * 10 - 20, n)
+        p.px[-1], p.py[-1] = cells_x * 10 - 5, cells_y * 10 - 5
+        p.volume[:] = 25.0
+        p.materials = [WATER]
+        p.material[:] = 0
+        config = {"grid": {"cellsX": cells_x, "cellsY": cells_y, "cellSize": 10}, "particleMass": 0.5,
+                  "particleVolume": 25.0, "material": WATER}
+        runs = []
+        for fused in (False, True):
+            solver = create_mpm_mls_gpu_solver(p, config)
+            try:
+                solver.set_substep_variant(fused=fused, p2g_records=False)
+                solver.step_batch(5, 1 / 1500, {"x": 3.0, "y": 90.0})
+                assert solver.read_status_words()[0] == 0
+                runs.append(solver.read_particles_packed()[0])
+            finally:
+                solver.dispose()
+        assert np.array_equal(np.ascontiguousarray(runs[0]).view(np.uint32), np.ascontiguousarray(runs[1]).view(np.uint32))
