@@ -1031,12 +1031,13 @@ __global__ void k_tile_scatter(Ctx c)
 // more, a round then takes its chain of dependent instructions).
 // The last CTA to have read whether the scene runs starts the substep
 // (begin_substep).  What it costs is latency: the counts, keys and ranks come
-// in together, then the scan, then the stores.  A CTA has as few threads as
-// its barriers, scan and start are short with, of TILES tiles each: against 1,024
-// threads of 4 tiles a substep of 1,600 particles fell from 19.4 to 18.6 us, of
-// 20,011 (325 tiles) from 21.1 to 19.6, of 150,002 (1,056 tiles, 256 threads of
-// 8) from 29.2 to 28.2; 128 threads of 8 tiles 20.3 and 256 of 16 29.2 there
-// (two kernels instead of one: 0.6 us more).
+// in together, then the scan, then the stores.  Small CTAs start sooner and
+// wait less at barriers, so their threads are few, of TILES tiles each: against 1,024 threads of 4 tiles a substep of 1,600 particles fell
+// from 19.4 to 18.6 us, of 20,011 (325 tiles) from 21.1 to 19.6 (128 threads of
+// 8: 20.3), of 150,002 (1,056 tiles, 256 threads of 8) from 29.2 to 28.2 (512 of 8
+// 28.6, 256 of 16 29.2), of 240,000 (1,702 tiles, 256 of 8) from 36.2 to 35.7 (35.8,
+// 37.6).  At 2,046 tiles 0.3 us are left of it; at 2,730 (400,000 particles) the
+// many CTAs' scans of all tiles cost more than their starts: 512 of 8 46.2, 1,024 of 4 45.3.
 template <int THREADS, int TILES>
 __global__ void __launch_bounds__(THREADS) k_tile_bucket(Ctx c)
 {
@@ -3995,7 +3996,7 @@ __global__ void k_surface_decode(unsigned long long *acc, float2 *field, uint32_
 // the instances the host launches
 template __global__ void k_tile_bucket<256, 4>(Ctx);
 template __global__ void k_tile_bucket<256, 8>(Ctx);
-template __global__ void k_tile_bucket<512, 8>(Ctx);
+template __global__ void k_tile_bucket<1024, 4>(Ctx);
 // The trial deformation G2P computes (deformation_trial) for `n` given
 // (F, C) pairs: trial F, increment, determinant and substep count, or the
 // flags of a failed integration in `flags`.

@@ -132,7 +132,7 @@ constexpr int SCAN_CHUNK = SCAN_THREADS * SCAN_ITEMS;
 constexpr int SCAN_TOP_THREADS = 1024;
 constexpr int ALLOC_THREADS = 256;  // k_tile_alloc: 4 tiles per thread, 1024 per CTA
 constexpr int ALLOC_ITEMS = 4;
-constexpr uint32_t BUCKET_TILES = 4096;  // tiles k_tile_bucket takes at most (512 threads of 8)
+constexpr uint32_t BUCKET_TILES = 4096;  // tiles k_tile_bucket takes at most (1,024 threads of 4)
 constexpr uint32_t ALLOC_TILES = ALLOC_THREADS * ALLOC_ITEMS;
 
 // default P2G: the particles whose base node lies in one 16x8-node tile reach

@@ -537,10 +537,10 @@ void enqueue_substep(mpm_solver *s, int parity)
         mark(K_SUBSTEP);
     } else if (s->gather()) {
         if (buckets_at_once(s)) {
-            // the fewest threads whose tiles cover the scene's
+            // (the lines: see the kernel)
             const unsigned quads = (s->n + 3) / 4, n_tiles = s->scenes[0].tiles;
-            const unsigned threads = n_tiles <= 2048u ? 256u : 512u;
-            launch(s, n_tiles <= 1024u ? k_tile_bucket<256, 4> : (n_tiles <= 2048u ? k_tile_bucket<256, 8> : k_tile_bucket<512, 8>),
+            const unsigned threads = n_tiles <= 2048u ? 256u : 1024u;
+            launch(s, n_tiles <= 1024u ? k_tile_bucket<256, 4> : (n_tiles <= 2048u ? k_tile_bucket<256, 8> : k_tile_bucket<1024, 4>),
                    dim3(blocks_for(quads, threads)), dim3(threads), 0, c);
             mark(K_TILE_BUCKET);
         } else {
